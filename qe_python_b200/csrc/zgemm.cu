@@ -3,12 +3,15 @@
 //   C = alpha * op(A) * B + beta * C,   op(A) = A ("N") or A^H ("C")
 //
 // All matrices are column-major with explicit leading dimensions.  The
-// plain form runs in FP64 (complex128) on the FP64 pipes: a register-tiled
-// SIMT kernel (64 x 64 block tile, 4 x 4 complex micro tile per thread,
-// 16-deep K tiles double-buffered in shared memory).  Contractions over the
-// long plane-wave dimension (calbec beta^H psi, Davidson V^H HV) split K
-// across blocks; the partial tiles go to caller scratch and a second kernel
-// reduces them in a fixed order, so results are deterministic.
+// plain form (complex128) runs on the FP64 tensor pipe (mma.sync m8n8k4; a
+// tcgen05 kind for FP64 does not exist) fed by a cp.async ring; complex64
+// products too small for the split-TF32 tensor-core GEMM run on a
+// register-tiled FP32 SIMT kernel (64 x 64 block tile, 4 x 4 complex micro
+// tile per thread, 16-deep K tiles double-buffered in shared memory).
+// Contractions over the long plane-wave dimension (calbec beta^H psi,
+// Davidson V^H HV) split K across blocks; the partial tiles go to caller
+// scratch and a second kernel reduces them in a fixed order, so results are
+// deterministic.
 //
 // Reference calls replaced: projector_overlaps (ZGEMM ConjTrans/NoTrans,
 // qepy_pw/_native_fft.pyx:694-731), add_projector_product (ZGEMM beta=1,
@@ -145,6 +148,169 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, int 
         *c = v;
       }
     }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 products on the tensor pipe.
+//
+// Bound by the FP64 pipe, whose rate is the same for FMA and mma.sync
+// (measured 36.5 and 37.2 TFLOP/s): what the SIMT kernel lost to shared-memory
+// loads (8 per 64 FMAs, bank conflicts on the transposed stores) and issue
+// slots, one m8n8k4 instruction per 256 multiply-adds gives back.  Four warps
+// (2 x 2) share a BM x BN complex tile; a warp's 8-row and 8-column fragments
+// are single 16-byte loads (re and im together), and each 8 x 8 x 4 complex
+// product is four real ones, op(A)'s conjugation being a sign flip of the
+// imaginary fragment.  K advances in steps of kMmaK through kMmaStages
+// cp.async buffers (16-byte copies: one complex value, so any leading
+// dimension works; values past the edges are zero-filled).
+// Shared layouts: K-contiguous operands are rows of kMmaK values at a stride
+// of 12 (4 mod 8: the 2 rows x 4 k of a load phase cover all banks), the
+// M-contiguous A of op N is rows of BM values at a stride of BM + 2 (2 mod 8).
+// Measured against the SIMT kernel: the 23 847 x 184 x 184 rotation 0.373 ->
+// 0.250 ms (25.8 TFLOP/s), H|psi> of 256 bands on 64^3 1.895 -> 1.343 ms.
+constexpr int kMmaK = 8, kMmaStages = 4, kMmaThreads = 128, kMmaStride = kMmaK + 4;
+
+template <int BMT, int BNT, bool CONJ_A>
+struct MmaTile {
+  static constexpr int a_values = CONJ_A ? BMT * kMmaStride : kMmaK * (BMT + 2);
+  static constexpr int b_values = BNT * kMmaStride;
+  static constexpr size_t smem = sizeof(double2) * (size_t)kMmaStages * (a_values + b_values);
+};
+
+__device__ __forceinline__ void cp_async16(double2* dst, const double2* src, bool valid) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int bytes = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes)
+               : "memory");
+}
+
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// One block: the BM x BN tile of op(A) B at (tile_m, tile_n) over the K range
+// of slice blockIdx.y.  P == nullptr: C = alpha*acc + beta*C, else the partial
+// slice.  Tiles are numbered with n fastest, so the blocks that share rows of
+// a tall A run side by side.
+template <int BMT, int BNT, bool CONJ_A>
+__global__ void __launch_bounds__(kMmaThreads, 2) zgemm_mma_kernel(
+    int M, int N, int K, int kchunk, int ntiles, double2 alpha, const double2* __restrict__ A,
+    int64_t lda, const double2* __restrict__ B, int64_t ldb, double2 beta, double2* C,
+    int64_t ldc, double2* __restrict__ P) {
+  using S = MmaTile<BMT, BNT, CONJ_A>;
+  constexpr int TM = BMT / 16, TN = BNT / 16;  // 8 x 8 tiles per warp
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* as = reinterpret_cast<double2*>(smem_raw);
+  double2* bs = as + kMmaStages * S::a_values;
+  const int tile_m = blockIdx.x / ntiles, tile_n = blockIdx.x - tile_m * ntiles;
+  const int m0 = tile_m * BMT, n0 = tile_n * BNT;
+  const int kbeg = blockIdx.y * kchunk, kend = min(K, kbeg + kchunk);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int wm = (warp & 1) * (BMT / 2), wn = (warp >> 1) * (BNT / 2);
+  const int row = lane >> 2, quad = lane & 3;
+  const int steps = kend > kbeg ? (kend - kbeg + kMmaK - 1) / kMmaK : 0;
+
+  auto load = [&](int step) {
+    if (step < steps) {
+      const int slot = step % kMmaStages, k0 = kbeg + step * kMmaK;
+      double2* a = as + slot * S::a_values;
+      double2* b = bs + slot * S::b_values;
+#pragma unroll
+      for (int r = 0; r < BMT * kMmaK / kMmaThreads; ++r) {
+        const int i = t + r * kMmaThreads;
+        const int k = CONJ_A ? i % kMmaK : i / BMT, m = CONJ_A ? i / kMmaK : i % BMT;
+        const bool valid = k0 + k < kend && m0 + m < M;
+        const double2* src = CONJ_A ? A + (k0 + k) + (int64_t)(m0 + m) * lda
+                                    : A + (m0 + m) + (int64_t)(k0 + k) * lda;
+        cp_async16(a + (CONJ_A ? m * kMmaStride + k : k * (BMT + 2) + m), valid ? src : A, valid);
+      }
+#pragma unroll
+      for (int r = 0; r < BNT * kMmaK / kMmaThreads; ++r) {
+        const int i = t + r * kMmaThreads, k = i % kMmaK, n = i / kMmaK;
+        const bool valid = k0 + k < kend && n0 + n < N;
+        cp_async16(b + n * kMmaStride + k, valid ? B + (k0 + k) + (int64_t)(n0 + n) * ldb : B,
+                   valid);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  double re[TM][TN][2], im[TM][TN][2];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+
+#pragma unroll
+  for (int s = 0; s < kMmaStages - 1; ++s) load(s);
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kMmaStages - 2) : "memory");
+    __syncthreads();  // this step's values are in; the slot loaded next has been read
+    load(step + kMmaStages - 1);
+    const double2* a = as + (step % kMmaStages) * S::a_values;
+    const double2* b = bs + (step % kMmaStages) * S::b_values;
+#pragma unroll
+    for (int kk = 0; kk < kMmaK; kk += 4) {
+      double2 av[TM], bv[TN];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const int m = wm + 8 * i + row, k = kk + quad;
+        av[i] = a[CONJ_A ? m * kMmaStride + k : k * (BMT + 2) + m];
+      }
+#pragma unroll
+      for (int j = 0; j < TN; ++j) bv[j] = b[(wn + 8 * j + row) * kMmaStride + kk + quad];
+      // re += ar br, im += ar bi, then re -+ ai bi, im +- ai br: an
+      // accumulator is revisited only after all the others
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) mma_f64(re[i][j], av[i].x, bv[j].x);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) mma_f64(im[i][j], av[i].x, bv[j].y);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const double ai = CONJ_A ? av[i].y : -av[i].y;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) mma_f64(re[i][j], ai, bv[j].y);
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const double ai = CONJ_A ? -av[i].y : av[i].y;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) mma_f64(im[i][j], ai, bv[j].x);
+      }
+    }
+  }
+  const bool use_beta = beta.x != 0.0 || beta.y != 0.0;
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + wm + 8 * i + row;
+    if (gm >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int gn = n0 + wn + 8 * j + 2 * quad + c;
+        if (gn >= N) continue;
+        const double x = re[i][j][c], y = im[i][j][c];
+        if (P != nullptr) {
+          P[(int64_t)blockIdx.y * M * N + gm + (int64_t)gn * M] = make_double2(x, y);
+        } else {
+          double2* o = C + gm + (int64_t)gn * ldc;
+          double2 v = make_double2(alpha.x * x - alpha.y * y, alpha.x * y + alpha.y * x);
+          if (use_beta) {
+            const double2 old = *o;
+            v.x += beta.x * old.x - beta.y * old.y;
+            v.y += beta.x * old.y + beta.y * old.x;
+          }
+          *o = v;
+        }
+      }
   }
 }
 
@@ -349,6 +515,38 @@ int choose_splits(int M, int N, int K) {
   return s < 1 ? 1 : s;
 }
 
+// Tile of the FP64 tensor kernel: per dimension the edge of 64, 48 or 32 with
+// the least padding (the larger one on a tie: fewer loads per product).
+int mma_edge(int n) {
+  int best = 64, cost = (n + 63) / 64 * 64;
+  for (int e : {48, 32}) {
+    const int c = (n + e - 1) / e * e;
+    if (c < cost) best = e, cost = c;
+  }
+  return best;
+}
+
+// K slices of the FP64 tensor kernel: the blocks of one SM share its FP64
+// pipe, so the time is that of the SM with the most tiles (at kSmRate
+// complex multiply-adds per microsecond), plus writing and reading the
+// partial slices; slices are at least 64 deep.  The rates only weigh the two
+// terms against each other.
+int mma_splits(int M, int N, int K) {
+  constexpr double kSmRate = 30.0e3, kSliceBytes = 4.0e6;  // per SM; bytes per us
+  const int bm = mma_edge(M), bn = mma_edge(N);
+  const int64_t tiles = (int64_t)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+  int best = 1;
+  double best_time = 0.0;
+  for (int s = 1; s <= 64 && (s == 1 || K / s >= 64); ++s) {
+    const int64_t per_sm = (tiles * s + sm_count() - 1) / sm_count();
+    const int depth = ((K + s - 1) / s + kMmaK - 1) / kMmaK * kMmaK;
+    double time = (double)per_sm * depth * bm * bn / kSmRate;
+    if (s > 1) time += 2.0 + 32.0 * s * M * N / kSliceBytes;  // a second launch, slices out and in
+    if (s == 1 || time < 0.98 * best_time) best = s, best_time = time;
+  }
+  return best;
+}
+
 // Skinny OP_C plan: the narrow side (N, else M when N is wide), the large
 // side Mb and the number of K slices (about four waves, each >= 1024 deep).
 struct SkinnyC {
@@ -436,6 +634,39 @@ int gemm_skinny_n(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, co
   return qeb::cuda_status(cudaGetLastError(), "zgemm skinny launch");
 }
 
+template <int BMT, int BNT, bool CONJ_A>
+int launch_mma_tile(int M, int N, int K, int kchunk, int splits, double2 al, const double2* A,
+                    int64_t lda, const double2* B, int64_t ldb, double2 be, double2* C,
+                    int64_t ldc, double2* partials, cudaStream_t stream) {
+  auto* kernel = zgemm_mma_kernel<BMT, BNT, CONJ_A>;
+  constexpr size_t smem = MmaTile<BMT, BNT, CONJ_A>::smem;
+  const cudaError_t e = qeb::raise_smem_limit(kernel, smem);
+  if (e != cudaSuccess) return qeb::cuda_status(e, "zgemm shared-memory limit");
+  const int mt = (M + BMT - 1) / BMT, nt = (N + BNT - 1) / BNT;
+  if ((int64_t)mt * nt > 0x7fffffff) {
+    qeb::set_error("zgemm: matrix too large for one launch");
+    return QEB_EUNSUPPORTED;
+  }
+  kernel<<<dim3(mt * nt, splits), kMmaThreads, smem, stream>>>(M, N, K, kchunk, nt, al, A, lda, B,
+                                                               ldb, be, C, ldc, partials);
+  return QEB_OK;
+}
+
+template <class... Args>
+int launch_mma(int opa, int M, int N, Args... args) {
+  const int bm = mma_edge(M), bn = mma_edge(N);
+  const bool conj = opa == QEB_OP_C;
+#define QEB_TILE(m, n)                                                              \
+  if (bm == m && bn == n)                                                           \
+    return conj ? launch_mma_tile<m, n, true>(M, N, args...)                        \
+                : launch_mma_tile<m, n, false>(M, N, args...);
+  QEB_TILE(64, 64) QEB_TILE(64, 48) QEB_TILE(64, 32)
+  QEB_TILE(48, 64) QEB_TILE(48, 48) QEB_TILE(48, 32)
+  QEB_TILE(32, 64) QEB_TILE(32, 48) QEB_TILE(32, 32)
+#undef QEB_TILE
+  return QEB_EUNSUPPORTED;
+}
+
 template <typename T>
 int gemm(int opa, int M, int N, int K, const double* alpha, const void* A, int64_t lda,
          const void* B, int64_t ldb, const double* beta, void* C, int64_t ldc, void* scratch,
@@ -465,38 +696,38 @@ int gemm(int opa, int M, int N, int K, const double* alpha, const void* A, int64
     return gemm_skinny_n<T>(M, N, K, al, static_cast<const C2<T>*>(A), lda,
                             static_cast<const C2<T>*>(B), ldb, be, static_cast<C2<T>*>(C), ldc,
                             stream);
-  const size_t smem = sizeof(Tile<T>);
-  static bool configured[2] = {false, false};
-  if (!configured[opa]) {
-    cudaFuncSetAttribute(gemm_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    cudaFuncSetAttribute(gemm_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    configured[opa] = true;
-  }
-  int splits = (opa == QEB_OP_C) ? choose_splits(M, N, K) : 1;
+  constexpr bool kMma = sizeof(T) == 8;
+  int splits = (opa == QEB_OP_C) ? (kMma ? mma_splits(M, N, K) : choose_splits(M, N, K)) : 1;
   const int64_t slice_bytes = (int64_t)M * N * (int64_t)sizeof(C2<T>);
   if (splits > 1) {
     const int64_t fit = (scratch == nullptr) ? 0 : scratch_bytes / slice_bytes;
     if (fit < splits) splits = (int)(fit < 1 ? 1 : fit);
   }
+  constexpr int kStep = kMma ? kMmaK : BK;
   int kchunk = K;
   if (splits > 1) {
     kchunk = (K + splits - 1) / splits;
-    kchunk = (kchunk + BK - 1) / BK * BK;
+    kchunk = (kchunk + kStep - 1) / kStep * kStep;
     splits = (K + kchunk - 1) / kchunk;
   }
   if (K == 0) kchunk = 1;
-  const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, splits);
   C2<T>* partials = (splits > 1) ? static_cast<C2<T>*>(scratch) : nullptr;
-  if (opa == QEB_OP_C) {
-    gemm_kernel<T, true><<<grid, THREADS, smem, stream>>>(
-        M, N, K, kchunk, al, static_cast<const C2<T>*>(A), lda, static_cast<const C2<T>*>(B),
-        ldb, be, static_cast<C2<T>*>(C), ldc, partials);
+  if constexpr (kMma) {
+    const int rc = launch_mma(opa, M, N, K, kchunk, splits, make_double2(al.re, al.im),
+                              static_cast<const double2*>(A), lda,
+                              static_cast<const double2*>(B), ldb, make_double2(be.re, be.im),
+                              static_cast<double2*>(C), ldc,
+                              reinterpret_cast<double2*>(partials), stream);
+    if (rc) return rc;
   } else {
-    gemm_kernel<T, false><<<grid, THREADS, smem, stream>>>(
-        M, N, K, kchunk, al, static_cast<const C2<T>*>(A), lda, static_cast<const C2<T>*>(B),
-        ldb, be, static_cast<C2<T>*>(C), ldc, partials);
+    const size_t smem = sizeof(Tile<T>);
+    const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, splits);
+    auto* kernel = opa == QEB_OP_C ? gemm_kernel<T, true> : gemm_kernel<T, false>;
+    const cudaError_t e = qeb::raise_smem_limit(kernel, smem);
+    if (e != cudaSuccess) return qeb::cuda_status(e, "cgemm shared-memory limit");
+    kernel<<<grid, THREADS, smem, stream>>>(
+        M, N, K, kchunk, al, static_cast<const C2<T>*>(A), lda, static_cast<const C2<T>*>(B), ldb,
+        be, static_cast<C2<T>*>(C), ldc, partials);
   }
   qeb::count_launches(splits > 1 ? 2 : 1);
   if (splits > 1) {
@@ -518,7 +749,7 @@ extern "C" int64_t qeb_zgemm_scratch_bytes(int opa, int M, int N, int K, int pre
     const SkinnyC p = skinny_c_plan(M, N, K);
     return p.splits > 1 ? (int64_t)p.splits * p.mb * p.ns * elem : 0;
   }
-  const int splits = choose_splits(M, N, K);
+  const int splits = precision == QEB_F64 ? mma_splits(M, N, K) : choose_splits(M, N, K);
   return splits > 1 ? (int64_t)splits * M * N * elem : 0;
 }
 
