@@ -73,7 +73,8 @@ int qeb_local_plan_create(qeb_local_plan** plan, int nx, int ny, int nz, int64_t
                           const int64_t* z_major_slots, int precision);
 int qeb_local_plan_destroy(qeb_local_plan* plan);
 /* info[0..7] = nx, ny, nz, npw, sticks, active y rows, precision, device;
- * with n >= 9, info[8] = K of the pruned plane pass (0: active-row plane). */
+ * with n >= 9, info[8] = blocks at each end of x and y that the compile-time
+ * plane kernel keeps (0: run-time plane kernel). */
 int qeb_local_plan_info(const qeb_local_plan* plan, int64_t* info, int n);
 /* Bytes of caller scratch needed for nbands (the stick buffer
  * nbands*nz*sticks complex values); the role of the grid scratch argument
@@ -102,7 +103,7 @@ int qeb_apply_local_profiled(const qeb_local_plan* plan, void* scratch, int64_t 
  * stick buffers are carved from one scratch of qeb_local_multi_scratch_bytes()
  * bytes.  Chosen-form batching of the per-k apply_serial_spatial calls of
  * qepy_pw/pw/scf.py:3396-3411 (no counterpart in the reference).  Grids
- * without a four-step factorisation run one launch sequence per k point. */
+ * without line transforms run one launch sequence per k point. */
 int64_t qeb_local_multi_scratch_bytes(int nk, const qeb_local_plan* const* plans,
                                       const int64_t* nbands);
 int qeb_apply_local_multi(int nk, const qeb_local_plan* const* plans, void* scratch,
@@ -111,8 +112,8 @@ int qeb_apply_local_multi(int nk, const qeb_local_plan* const* plans, void* scra
                           const void* const* kinetic, void* const* out, const int64_t* ld_out,
                           void* stream);
 
-/* Process-wide choice of how the four-step passes run (qeb_apply_local and
- * qeb_apply_local_multi on cubic grids): 0 (default) three launches, one
+/* Process-wide choice of how the line-transform passes run (qeb_apply_local and
+ * qeb_apply_local_multi): 0 (default) three launches, one
  * per pass; 1 one persistent cooperative launch that runs the three passes
  * of every k point with a grid barrier between them (the barrier's words
  * are the last 256 bytes of the caller's scratch; a barrier that gives up
@@ -124,7 +125,10 @@ int qeb_persistent_passes(void);
 /* density[(x*ny + y)*nz + z] += sum_b weights[b] |FFT^+(psi[:, b])(x,y,z)|^2
  * (float64 accumulation; weights is a device float64 array of nbands).
  * Replaces accumulate_density_serial(_spatial)
- * (qepy_pw/_native_fft.pyx:2537-2648; operator at :137-193). */
+ * (qepy_pw/_native_fft.pyx:2537-2648; operator at :137-193).  With scratch of
+ * qeb_density_scratch_bytes the bands are added in a grid of their own there
+ * first; qeb_local_scratch_bytes is enough (slower for many bands). */
+int64_t qeb_density_scratch_bytes(const qeb_local_plan* plan, int64_t nbands);
 int qeb_accumulate_density(const qeb_local_plan* plan, void* scratch, int64_t scratch_bytes,
                            const void* psi, int64_t ld_psi, int64_t nbands,
                            const double* weights, double* density, void* stream);

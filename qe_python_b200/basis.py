@@ -398,8 +398,8 @@ class LocalPotentialWorkspace:
                    lib.qeb_local_plan_info(self._plan, info.ctypes.data, 9))
         self.stick_count = int(info[4])
         self.active_rows = int(info[5])
-        # K of the pruned plane pass (every stick within the 2 K N2 kept rows
-        # and columns of a 64-point plane), 0 for the active-row plane
+        # blocks at each end of x and y that the compile-time plane kernel of a
+        # square plane keeps (qeb_local_plan.line_k), 0 for the run-time kernel
         self.pruned_plane = int(info[8])
         self._potential_cache: tuple | None = None
         self._kinetic_cache: tuple | None = None
@@ -556,7 +556,8 @@ class LocalPotentialWorkspace:
         batch = min(max(batch, 1), 65535)
         for start in range(0, nb, batch):
             count = min(batch, nb - start)
-            scratch, nbytes = self._scratch(count)
+            nbytes = int(lib.qeb_density_scratch_bytes(self._plan, count))
+            scratch = self.scratch_pool.buffer("sticks", nbytes, self.device)
             status = lib.qeb_accumulate_density(
                 self._plan, scratch.data_ptr(), nbytes,
                 vectors.data_ptr() + start * ld * elem, ld, count,
@@ -591,7 +592,7 @@ _MULTI_SCRATCH = FFTScratchPool()
 
 
 def set_persistent_passes(enabled: bool) -> None:
-    """Run the three four-step passes of a local apply (one k point or a
+    """Run the three line-transform passes of a local apply (one k point or a
     batch) as one persistent cooperative launch with grid barriers between
     them (True), or as three launches (False, the default).  Process-wide;
     the arithmetic is the same either way (qeb_set_persistent_passes)."""

@@ -214,10 +214,15 @@ const C2<T>* tw_ptr(const qeb_local_plan* p, int which) {
 
 // Scratch of one apply: the stick buffer (nbands x nz x nst values), rounded
 // up to 256 bytes, then the 256-byte word block of the persistent launch's
-// grid barrier (local_fast.cu).
+// grid barrier (local_lines.cu).
 static int64_t stick_region_bytes(const qeb_local_plan* p, int64_t nbands) {
   const int64_t elem = (p->precision == QEB_F64) ? 16 : 8;
   return (nbands * (int64_t)p->nz * p->nst * elem + 255) / 256 * 256;
+}
+
+static unsigned int* barrier_words(const qeb_local_plan* p, void* sticks, int64_t nbands) {
+  return reinterpret_cast<unsigned int*>(static_cast<unsigned char*>(sticks) +
+                                         stick_region_bytes(p, nbands));
 }
 
 template <typename T>
@@ -229,10 +234,15 @@ int launch_apply(const qeb_local_plan* p, C2<T>* sticks, const C2<T>* psi, int64
     qeb::set_error("apply_local: at most 65535 bands per call (got %lld)", (long long)nb);
     return QEB_EINVAL;
   }
-  if (p->fast_xy >= 0 && p->fast_z >= 0)
-    return qeb::fast_apply(p, sticks, psi, ld, nb, potential, kinetic, out, ldo, stream, events,
-                           reinterpret_cast<unsigned int*>(reinterpret_cast<unsigned char*>(sticks) +
-                                                           stick_region_bytes(p, nb)));
+  if (p->lines) {
+    const qeb_local_plan* plans[1] = {p};
+    void* st[1] = {sticks};
+    void* o[1] = {out};
+    const void* ps[1] = {psi};
+    const void* kin[1] = {kinetic};
+    return qeb::lines_apply(1, plans, st, ps, &ld, &nb, potential, kin, o, &ldo, stream, events,
+                            barrier_words(p, sticks, nb));
+  }
   const dim3 grid_ac((p->nst + kSticksPerBlock - 1) / kSticksPerBlock, (unsigned)nb);
   const dim3 grid_b(p->nz, (unsigned)nb);
   if (events) cudaEventRecord(events[0], stream);
@@ -255,15 +265,16 @@ int launch_apply(const qeb_local_plan* p, C2<T>* sticks, const C2<T>* psi, int64
 }
 
 template <typename T>
-int launch_density(const qeb_local_plan* p, C2<T>* sticks, const C2<T>* psi, int64_t ld,
-                   int64_t nb, const double* weights, double* density, cudaStream_t stream) {
+int launch_density(const qeb_local_plan* p, C2<T>* sticks, double* grid, const C2<T>* psi,
+                   int64_t ld, int64_t nb, const double* weights, double* density,
+                   cudaStream_t stream) {
   if (nb == 0) return QEB_OK;
   if (nb > 65535) {
     qeb::set_error("accumulate_density: at most 65535 bands per call (got %lld)", (long long)nb);
     return QEB_EINVAL;
   }
-  if (p->fast_xy >= 0 && p->fast_z >= 0)
-    return qeb::fast_density(p, sticks, psi, ld, nb, weights, density, stream);
+  if (p->lines)
+    return qeb::lines_density(p, sticks, grid, psi, ld, nb, weights, density, stream);
   const dim3 grid_ac((p->nst + kSticksPerBlock - 1) / kSticksPerBlock, (unsigned)nb);
   const dim3 grid_b(p->nz, (unsigned)nb);
   pass_a_kernel<T><<<grid_ac, kThreads, pass_ac_smem<T>(p), stream>>>(
@@ -296,8 +307,9 @@ void free_plan(qeb_local_plan* p) {
   cudaFree(p->stick_pos);
   cudaFree(p->ay_to_y);
   cudaFree(p->y_to_ay);
-  cudaFree(p->slot_pos);
-  cudaFree(p->ay_to_slot);
+  cudaFree(p->entry_pos);
+  cudaFree(p->stick_map);
+
   cudaFree(p->tw);
   delete p;
 }
@@ -369,7 +381,8 @@ extern "C" int qeb_local_plan_create(qeb_local_plan** out, int nx, int ny, int n
       return QEB_EINVAL;
     }
     zs[g] = (int32_t)(slot / plane);
-    xy[g] = slot % plane;
+    // stick key: y-major, so that the sticks of one y follow one another in x
+    xy[g] = (slot % plane) % ny * nx + (slot % plane) / ny;
   }
   std::vector<int64_t> sticks(xy);
   std::sort(sticks.begin(), sticks.end());
@@ -407,7 +420,7 @@ extern "C" int qeb_local_plan_create(qeb_local_plan** out, int nx, int ny, int n
   }
   // Active y rows.
   std::vector<int32_t> y_to_ay(ny, -1), ay_to_y;
-  for (int s = 0; s < nst; ++s) y_to_ay[sticks[s] % ny] = 1;
+  for (int s = 0; s < nst; ++s) y_to_ay[sticks[s] / nx] = 1;
   for (int y = 0; y < ny; ++y) {
     if (y_to_ay[y] >= 0) {
       y_to_ay[y] = (int32_t)ay_to_y.size();
@@ -418,53 +431,51 @@ extern "C" int qeb_local_plan_create(qeb_local_plan** out, int nx, int ny, int n
   p->nx_pad = odd_pad(nx);
   p->ny_pad = odd_pad(ny);
   p->nz_pad = odd_pad(nz);
-  // Four-step kernels when both the plane (nx == ny) and the z lines have a
-  // listed factorisation; QEB_FORCE_GENERIC=1 selects the Stockham kernels.
-  const char* force_generic = std::getenv("QEB_FORCE_GENERIC");
-  p->fast_xy = (nx == ny) ? qeb::four_variant(nx) : -1;
-  p->fast_z = qeb::four_variant(nz);
-  if (p->fast_xy < 0 || p->fast_z < 0 || (force_generic && force_generic[0] == '1')) {
-    p->fast_xy = -1;
-    p->fast_z = -1;
-  }
   std::vector<int32_t> stick_pos(nst);
   for (int s = 0; s < nst; ++s) {
-    const int x = (int)(sticks[s] / ny), y = (int)(sticks[s] % ny);
+    const int x = (int)(sticks[s] % nx), y = (int)(sticks[s] / nx);
     stick_pos[s] = y_to_ay[y] * p->nx_pad + x;
   }
-  p->zmask = 0xffffffffu;
-  int n1 = 0, n2 = 0;
-  if (p->fast_z >= 0 && qeb::four_split(p->fast_z, &n1, &n2)) {
-    uint32_t m = 0;
-    for (int64_t e = 0; e < npw; ++e) m |= 1u << (entry_z[e] / n2);
-    p->zmask = m;
-  }
-  // Pruned plane: every stick's x and y within the 2 K N2 kept rows.
-  p->prune_k = 0;
-  std::vector<int32_t> slot_pos, ay_to_slot;
+  // Line transforms: kept blocks and the stick lookup; QEB_FORCE_GENERIC=1
+  // selects the Stockham kernels, QEB_PRUNE_PLANE=0 the run-time plane kernel.
+  const char* force_generic = std::getenv("QEB_FORCE_GENERIC");
   const char* prune_env = std::getenv("QEB_PRUNE_PLANE");
-  const int prune_k = p->fast_xy >= 0 ? qeb::prune_k_of(p->fast_xy) : 0;
-  if (prune_k > 0 && !(prune_env && prune_env[0] == '0') &&
-      qeb::four_split(p->fast_xy, &n1, &n2)) {
-    const int half = prune_k * n2, gap = nx - 2 * half;
-    auto kept = [&](int c) { return c < half || c >= nx - half; };
-    bool fits = 2 * prune_k < n1;
-    for (int s = 0; s < nst && fits; ++s)
-      fits = kept((int)(sticks[s] / ny)) && kept((int)(sticks[s] % ny));
-    if (fits) {
-      auto slot = [&](int y) { return y < half ? y : y - gap; };
-      slot_pos.resize(nst);
-      for (int s = 0; s < nst; ++s) {
-        const int x = (int)(sticks[s] / ny), y = (int)(sticks[s] % ny);
-        slot_pos[s] = slot(y) * p->nx_pad + x;
-      }
-      for (int y : ay_to_y) ay_to_slot.push_back(slot(y));
-      p->prune_k = prune_k;
+  std::vector<int32_t> stick_map, entry_pos;
+  int x1, x2, y1, y2, z1, z2;
+  if (qeb::line_split(nx, &x1, &x2) && qeb::line_split(ny, &y1, &y2) &&
+      qeb::line_split(nz, &z1, &z2) && !(force_generic && force_generic[0] == '1')) {
+    int reach = 0;
+    auto from_end = [](int c, int n) { return std::min(c + 1, n - c); };
+    for (int s = 0; s < nst; ++s) {
+      const int x = (int)(sticks[s] % nx), y = (int)(sticks[s] / nx);
+      reach = std::max(reach, std::max(from_end(x, nx), from_end(y, ny)));
+      p->xmask |= 1u << (x / x2);
+      p->ymask |= 1u << (y / y2);
     }
+    if (nx == ny && !(prune_env && prune_env[0] == '0')) p->line_k = qeb::line_keep(nx, reach);
+    if (p->line_k > 0) {
+      p->xmask = 0;
+      for (int i = 0; i < x1; ++i)
+        if (i < p->line_k || i >= x1 - p->line_k) p->xmask |= 1u << i;
+      p->ymask = p->xmask;
+    }
+    std::vector<int> row(nx, -1);
+    for (int x = 0; x < nx; ++x)
+      if ((p->xmask >> (x / x2)) & 1u) row[x] = p->line_rows++;
+    stick_map.assign((size_t)ny * p->line_rows, -1);
+    for (int s = 0; s < nst; ++s)
+      stick_map[(size_t)(sticks[s] / nx) * p->line_rows + row[sticks[s] % nx]] = s;
+    entry_pos.resize(npw);
+    for (int64_t e = 0; e < npw; ++e) {
+      entry_pos[e] = entry_stick[e] % 32 * (nz | 1) + entry_z[e];
+      p->zmask |= 1u << (entry_z[e] / z2);
+    }
+    p->line_columns = qeb::line_columns(p);
+    p->lines = p->line_columns > 0;
   }
   int rc = QEB_OK;
-  if (p->prune_k > 0 &&
-      ((rc = upload(&p->slot_pos, slot_pos)) || (rc = upload(&p->ay_to_slot, ay_to_slot)))) {
+  if (p->lines && ((rc = upload(&p->stick_map, stick_map)) ||
+                   (rc = upload(&p->entry_pos, entry_pos)))) {
     free_plan(p);
     return rc;
   }
@@ -495,7 +506,7 @@ extern "C" int qeb_local_plan_create(qeb_local_plan** out, int nx, int ny, int n
     rc = upload(reinterpret_cast<C2<float>**>(&p->tw), tw);
     if (rc == QEB_OK) rc = set_smem_limits<float>(p);
   }
-  if (rc == QEB_OK && p->fast_xy >= 0) rc = qeb::fast_smem_limits(p);
+  if (rc == QEB_OK && p->lines) rc = qeb::lines_prepare(p);
   if (rc != QEB_OK) {
     free_plan(p);
     return rc;
@@ -522,13 +533,29 @@ extern "C" int qeb_local_plan_info(const qeb_local_plan* p, int64_t* info, int n
   info[5] = p->nay;
   info[6] = p->precision;
   info[7] = p->device;
-  if (n >= 9) info[8] = p->prune_k;
+  if (n >= 9) info[8] = p->line_k;
   return QEB_OK;
 }
 
 extern "C" int64_t qeb_local_scratch_bytes(const qeb_local_plan* p, int64_t nbands) {
   if (p == nullptr || nbands < 0) return -1;
   return stick_region_bytes(p, nbands) + 256;
+}
+
+// Bytes of the density grid that accumulate_density adds the bands in before
+// it adds the grid to the density (local_lines.cu), for enough points that the
+// scattered atomics cost more than the two extra launches: 24 bands on 36^3
+// (1.1 M) 29 us scattered, 33 us with the grid; 6 bands on 90^3 (4.4 M) 56 and
+// 55 us; 16 bands on 90^3 107 and 93 us.
+constexpr int64_t kDensityGridPoints = 4000000;
+static int64_t density_grid_bytes(const qeb_local_plan* p, int64_t nbands) {
+  const int64_t points = (int64_t)p->nx * p->ny * p->nz;
+  return p->lines && nbands * points >= kDensityGridPoints ? points * 8 : 0;
+}
+
+extern "C" int64_t qeb_density_scratch_bytes(const qeb_local_plan* p, int64_t nbands) {
+  if (p == nullptr || nbands < 0) return -1;
+  return qeb_local_scratch_bytes(p, nbands) + density_grid_bytes(p, nbands);
 }
 
 static int check_call(const qeb_local_plan* p, const void* scratch, int64_t scratch_bytes,
@@ -618,7 +645,7 @@ extern "C" int qeb_apply_local_multi(int nk, const qeb_local_plan* const* plans,
     return need < 0 ? QEB_EINVAL : QEB_ESCRATCH;
   }
   const qeb_local_plan* p0 = plans[0];
-  bool fused = p0 != nullptr && p0->fast_xy >= 0 && p0->fast_z >= 0;
+  bool fused = true;  // every k point by line transforms
   void* sticks[QEB_MAX_KBATCH];
   unsigned char* cursor = static_cast<unsigned char*>(scratch);
   for (int k = 0; k < nk; ++k) {
@@ -639,19 +666,15 @@ extern "C" int qeb_apply_local_multi(int nk, const qeb_local_plan* const* plans,
       qeb::set_error("apply_local_multi: every k point must use the same grid, precision and device");
       return QEB_EINVAL;
     }
-    fused = fused && p->fast_xy == p0->fast_xy && p->fast_z == p0->fast_z &&
-            p->nx_pad == p0->nx_pad && p->nz_pad == p0->nz_pad;
+    fused = fused && p->lines;
     sticks[k] = cursor;
     cursor += round_up_256(qeb_local_scratch_bytes(p, nbands[k]));
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (fused)
-    return qeb::fast_apply_multi(nk, plans, sticks, psi, ld_psi, nbands, potential_native, kinetic,
-                                 out, ld_out, s,
-                                 reinterpret_cast<unsigned int*>(
-                                     static_cast<unsigned char*>(sticks[0]) +
-                                     stick_region_bytes(plans[0], nbands[0])));
-  // grids without a four-step variant: one launch sequence per k point
+    return qeb::lines_apply(nk, plans, sticks, psi, ld_psi, nbands, potential_native, kinetic, out,
+                            ld_out, s, nullptr, barrier_words(plans[0], sticks[0], nbands[0]));
+  // grids without line transforms: one launch sequence per k point
   for (int k = 0; k < nk; ++k) {
     const int rc = qeb_apply_local(plans[k], sticks[k],
                                    qeb_local_scratch_bytes(plans[k], nbands[k]), psi[k],
@@ -673,12 +696,16 @@ extern "C" int qeb_accumulate_density(const qeb_local_plan* p, void* scratch,
     return QEB_EINVAL;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  double* grid = nullptr;
+  if (density_grid_bytes(p, nbands) > 0 && scratch_bytes >= qeb_density_scratch_bytes(p, nbands))
+    grid = reinterpret_cast<double*>(static_cast<unsigned char*>(scratch) +
+                                     qeb_local_scratch_bytes(p, nbands));
   if (p->precision == QEB_F64) {
-    return launch_density<double>(p, static_cast<C2<double>*>(scratch),
+    return launch_density<double>(p, static_cast<C2<double>*>(scratch), grid,
                                   static_cast<const C2<double>*>(psi), ld, nbands, weights,
                                   density, s);
   }
-  return launch_density<float>(p, static_cast<C2<float>*>(scratch),
+  return launch_density<float>(p, static_cast<C2<float>*>(scratch), grid,
                                static_cast<const C2<float>*>(psi), ld, nbands, weights, density,
                                s);
 }

@@ -1,0 +1,8 @@
+// The plane pass in FP64 (local_lines.cuh).
+#include "local_plane_launch.cuh"
+
+int qeb::lines::plane_pass(const KBatch<double>& kb, const qeb_local_plan* p, int mode, int nk, int nb,
+                           const double* potential, const DensityTarget& rho, cudaStream_t s) {
+  return mode == 0 ? launch_plane<double, 0>(kb, p, nk, nb, potential, rho, s)
+                   : launch_plane<double, 1>(kb, p, nk, nb, potential, rho, s);
+}
