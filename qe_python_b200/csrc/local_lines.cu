@@ -3,7 +3,7 @@
 #include <algorithm>
 #include <atomic>
 
-#include "line_lengths.h"
+#include "line_lengths.cuh"
 #include "local_lines.cuh"
 #include "../../include/qe_b200.h"
 

@@ -79,7 +79,7 @@ struct KBatch {
 };
 
 // Factors and sizes of the plane (z lines): compile-time for the cubic
-// lengths of line_lengths.h, run-time otherwise.  keep_x(d, i): whether block
+// lengths of line_lengths.cuh, run-time otherwise.  keep_x(d, i): whether block
 // i of x holds a stick, row_block(i): its place among the kept blocks.
 template <int N1, int N2, int K, int COLUMNS>
 struct StaticPlane {

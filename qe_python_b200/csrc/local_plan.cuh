@@ -22,7 +22,7 @@ struct qeb_local_plan {
   int device;
   qeb::FftDesc fx, fy, fz;
   // Line transforms: every axis has a two-factor split n = n1 n2
-  // (line_lengths.h) and the plane fits shared memory; else the generic
+  // (line_lengths.cuh) and the plane fits shared memory; else the generic
   // kernels run.
   bool lines;
   // Static plane kernel of square planes whose sticks all lie in

@@ -5,7 +5,7 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include "line_lengths.h"
+#include "line_lengths.cuh"
 #include "local_lines.cuh"
 #include "../../include/qe_b200.h"
 
