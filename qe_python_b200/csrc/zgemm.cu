@@ -18,6 +18,7 @@
 // :782-836), the Davidson reduced-matrix and Ritz products
 // (qepy_pw/diagonalization.py:658-726) and coupling @ overlaps (:348).
 #include <mutex>
+#include <type_traits>
 
 #include "qeb_common.cuh"
 #include "../../include/qe_b200.h"
@@ -341,85 +342,114 @@ __global__ void reduce_partials(int M, int N, int splits, const C2<T>* __restric
 
 constexpr int kSkinnyMax = 16;
 constexpr int kSkinnyThreads = 256;
-constexpr int kSkinnyColumns = kSkinnyThreads / 32;  // large-operand columns per block (OP_C)
-constexpr int kSkinnyChunkC = 128;                   // K rows staged per step (OP_C)
-constexpr int kSkinnyChunkN = 64;                    // K rows staged per step (OP_N)
+constexpr int kSkinnyWarps = kSkinnyThreads / 32;
+constexpr int kSkinnyRows = 64;  // rows per block (OP_N), two per lane
 
-int skinny_width(int n) { return n <= 4 ? 4 : (n <= 8 ? 8 : 16); }
+// Columns of the large operand per warp (OP_C): each narrow value loaded
+// serves that many of its multiply-adds.
+constexpr int skinny_cols(int ns) { return ns <= 8 ? 4 : 2; }
 
-// D[mb, ns] = sum_k conj(X[k, mb]) Y[k, ns] over this block's K range, one
-// warp per large column mb, Y rows staged [ns][k].  splits == 1: the block
-// writes C directly; else the partial slice blockIdx.y of P (Mb x Ns).
+// V consecutive values from p; `full` says that all of them are inside.
+template <typename T, int V>
+__device__ __forceinline__ void load_run(C2<T> (&v)[V], const C2<T>* __restrict__ p, bool full) {
+  if constexpr (V == 2) {  // two complex64 values in one 16-byte load
+    if (full) {
+      const float4 w = __ldg(reinterpret_cast<const float4*>(p));
+      v[0] = qeb::mk<T>(w.x, w.y);
+      v[1] = qeb::mk<T>(w.z, w.w);
+    } else {
+      v[0] = p[0];
+      v[1] = qeb::mk<T>(0, 0);
+    }
+  } else {
+    v[0] = p[0];
+  }
+}
+
+// D[mb, ns] = sum_k conj(X[k, mb]) Y[k, ns] over this block's K range.  A warp
+// owns MC columns of X and reads them with MC + NS loads per 4 MC NS
+// multiply-adds, lanes along k (one column per warp with Y staged in shared
+// memory was bound by its NS shared-memory loads per value of X: beta^H psi of
+// 5 bands, 80 725 x 864 complex64, 257 us).  WK warps share a column group and
+// split the K range between them (short products, whose few columns would
+// leave the loads of one warp in a chain).  splits == 1: the block writes C
+// directly; else the partial slice blockIdx.y of P (Mb x Ns).
 // Output mapping: swapped == 0: C[mb, ns] = alpha D + beta C;
 //                 swapped == 1: C[ns, mb] = alpha conj(D) + beta C.
-template <typename T, int NS>
+template <typename T, int NS, int V, int WK>
 __global__ void __launch_bounds__(kSkinnyThreads) skinny_c_kernel(
     int Mb, int Ns, int K, int krange, const C2<T>* __restrict__ X, int64_t ldx,
     const C2<T>* __restrict__ Y, int64_t ldy, C2<T> alpha, C2<T> beta, C2<T>* C, int64_t ldc,
     int swapped, C2<T>* __restrict__ P) {
-  __shared__ C2<T> ys[NS][kSkinnyChunkC];
+  constexpr int MC = skinny_cols(NS), WM = kSkinnyWarps / WK;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mb = blockIdx.x * kSkinnyColumns + warp;
+  const int m0 = (blockIdx.x * WM + warp / WK) * MC;
   const int kbeg = blockIdx.y * krange;
   const int kend = min(K, kbeg + krange);
-  const C2<T> zero = qeb::mk<T>(0, 0);
-  C2<T> acc[NS];
+  const C2<T>* x[MC];
+  const C2<T>* y[NS];
 #pragma unroll
-  for (int n = 0; n < NS; ++n) acc[n] = zero;
-  const C2<T>* xcol = X + (int64_t)(mb < Mb ? mb : 0) * ldx;
-  for (int k0 = kbeg; k0 < kend; k0 += kSkinnyChunkC) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < NS * kSkinnyChunkC; i += kSkinnyThreads) {
-      const int n = i / kSkinnyChunkC, kk = i - n * kSkinnyChunkC;
-      const int k = k0 + kk;
-      ys[n][kk] = (n < Ns && k < kend) ? Y[k + (int64_t)n * ldy] : zero;
-    }
-    __syncthreads();
-    if (mb < Mb) {
-      C2<T> xv[kSkinnyChunkC / 32];
+  for (int i = 0; i < MC; ++i) x[i] = X + (int64_t)min(m0 + i, Mb - 1) * ldx;
 #pragma unroll
-      for (int j = 0; j < kSkinnyChunkC / 32; ++j) {
-        const int k = k0 + lane + 32 * j;
-        xv[j] = (k < kend) ? xcol[k] : zero;
-      }
+  for (int n = 0; n < NS; ++n) y[n] = Y + (int64_t)min(n, Ns - 1) * ldy;
+  C2<T> acc[MC][NS];
 #pragma unroll
-      for (int j = 0; j < kSkinnyChunkC / 32; ++j) {
-        const int kk = lane + 32 * j;
+  for (int i = 0; i < MC; ++i)
 #pragma unroll
-        for (int n = 0; n < NS; ++n) {
-          const C2<T> y = ys[n][kk];
-          // conj(x) * y
-          acc[n].re = fma(xv[j].re, y.re, acc[n].re);
-          acc[n].re = fma(xv[j].im, y.im, acc[n].re);
-          acc[n].im = fma(xv[j].re, y.im, acc[n].im);
-          acc[n].im = fma(-xv[j].im, y.re, acc[n].im);
-        }
-      }
+    for (int n = 0; n < NS; ++n) acc[i][n] = qeb::mk<T>(0, 0);
+  if (m0 < Mb) {
+    for (int k = kbeg + ((warp % WK) * 32 + lane) * V; k < kend; k += WK * 32 * V) {
+      const bool full = k + V <= kend;
+      C2<T> xv[MC][V], yv[NS][V];
+#pragma unroll
+      for (int i = 0; i < MC; ++i) load_run<T, V>(xv[i], x[i] + k, full);
+#pragma unroll
+      for (int n = 0; n < NS; ++n) load_run<T, V>(yv[n], y[n] + k, full);
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int i = 0; i < MC; ++i)
+#pragma unroll
+          for (int n = 0; n < NS; ++n) {  // conj(x) * y
+            acc[i][n].re = fma(xv[i][v].re, yv[n][v].re, acc[i][n].re);
+            acc[i][n].re = fma(xv[i][v].im, yv[n][v].im, acc[i][n].re);
+            acc[i][n].im = fma(xv[i][v].re, yv[n][v].im, acc[i][n].im);
+            acc[i][n].im = fma(-xv[i][v].im, yv[n][v].re, acc[i][n].im);
+          }
     }
   }
+  C2<T> mine = qeb::mk<T>(0, 0);  // lane l: entry (l / NS, l % NS), then l + 32, ...
+  __shared__ C2<T> part[WK > 1 ? kSkinnyWarps : 1][MC * NS];
 #pragma unroll
-  for (int n = 0; n < NS; ++n) {
+  for (int i = 0; i < MC; ++i)
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      acc[n].re += __shfl_xor_sync(0xffffffffu, acc[n].re, off);
-      acc[n].im += __shfl_xor_sync(0xffffffffu, acc[n].im, off);
+    for (int n = 0; n < NS; ++n) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        acc[i][n].re += __shfl_xor_sync(0xffffffffu, acc[i][n].re, off);
+        acc[i][n].im += __shfl_xor_sync(0xffffffffu, acc[i][n].im, off);
+      }
+      if (lane == i * NS + n) mine = acc[i][n];
     }
+  static_assert(MC * NS <= 32, "one entry per lane");
+  if constexpr (WK > 1) {
+    if (lane < MC * NS) part[warp][lane] = mine;
+    __syncthreads();
+    if (warp % WK != 0) return;
+    if (lane < MC * NS)
+#pragma unroll
+      for (int w = 1; w < WK; ++w) mine = mine + part[warp + w][lane];
   }
-  if (lane != 0 || mb >= Mb) return;
-  const bool use_beta = beta.re != T(0) || beta.im != T(0);
-#pragma unroll
-  for (int n = 0; n < NS; ++n) {
-    if (n >= Ns) break;
-    if (P != nullptr) {
-      P[(int64_t)blockIdx.y * Mb * Ns + mb + (int64_t)n * Mb] = acc[n];
-    } else {
-      C2<T> d = acc[n];
-      if (swapped) d.im = -d.im;
-      C2<T>* c = swapped ? C + n + (int64_t)mb * ldc : C + mb + (int64_t)n * ldc;
-      C2<T> v = qeb::cmul(alpha, d);
-      if (use_beta) v = v + qeb::cmul(beta, *c);
-      *c = v;
-    }
+  const int mb = m0 + lane / NS, n = lane % NS;
+  if (lane >= MC * NS || mb >= Mb || n >= Ns) return;
+  if (P != nullptr) {
+    P[(int64_t)blockIdx.y * Mb * Ns + mb + (int64_t)n * Mb] = mine;
+  } else {
+    if (swapped) mine.im = -mine.im;
+    C2<T>* c = swapped ? C + n + (int64_t)mb * ldc : C + mb + (int64_t)n * ldc;
+    C2<T> v = qeb::cmul(alpha, mine);
+    if (beta.re != T(0) || beta.im != T(0)) v = v + qeb::cmul(beta, *c);
+    *c = v;
   }
 }
 
@@ -443,54 +473,79 @@ __global__ void skinny_reduce(int Mb, int Ns, int splits, const C2<T>* __restric
   }
 }
 
-// C[m, n] = alpha sum_k A[m, k] B[k, n] + beta C[m, n] for N <= NS: one
-// thread per row m, B rows staged [k][n] (every lane reads the same entry).
-template <typename T, int NS>
+// C[m, n] = alpha sum_k A[m, k] B[k, n] + beta C[m, n] for N <= NS.  A block
+// owns 64 rows, two per lane (V == 2: neighbouring complex64 rows in one
+// 16-byte load, else rows 32 apart), and its warps split K; the partial sums
+// meet in shared memory four columns at a time.  (One thread per row over the
+// whole of K left 2.1 blocks of 256 rows per SM on the 216-atom cell's
+// projector add, 80 725 x 864 x 5 complex64.)  With the kernel above: H|psi> of 5
+// bands of that cell 0.574 -> 0.409 ms.
+template <typename T, int NS, int V>
 __global__ void __launch_bounds__(kSkinnyThreads) skinny_n_kernel(
     int M, int N, int K, C2<T> alpha, const C2<T>* __restrict__ A, int64_t lda,
     const C2<T>* __restrict__ B, int64_t ldb, C2<T> beta, C2<T>* C, int64_t ldc) {
-  __shared__ C2<T> bs[kSkinnyChunkN][NS];
-  const int m = blockIdx.x * kSkinnyThreads + threadIdx.x;
-  const C2<T> zero = qeb::mk<T>(0, 0);
-  C2<T> acc[NS];
+  constexpr int kStep = 4;  // output columns reduced at a time
+  __shared__ C2<T> part[kSkinnyWarps][kStep][kSkinnyRows];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x * kSkinnyRows;
+  const int r0 = V == 2 ? 2 * lane : lane, r1 = V == 2 ? 2 * lane + 1 : lane + 32;
+  const int kper = (K + kSkinnyWarps - 1) / kSkinnyWarps;
+  const int kbeg = min(K, warp * kper), kend = min(K, kbeg + kper);
+  C2<T> acc[2][NS];
 #pragma unroll
-  for (int n = 0; n < NS; ++n) acc[n] = zero;
-  const C2<T>* arow = A + (m < M ? m : 0);
-  for (int k0 = 0; k0 < K; k0 += kSkinnyChunkN) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < NS * kSkinnyChunkN; i += kSkinnyThreads) {
-      const int n = i / kSkinnyChunkN, kk = i - n * kSkinnyChunkN;
-      const int k = k0 + kk;
-      bs[kk][n] = (n < N && k < K) ? B[k + (int64_t)n * ldb] : zero;
+  for (int n = 0; n < NS; ++n) acc[0][n] = acc[1][n] = qeb::mk<T>(0, 0);
+  const C2<T>* a0 = A + min(m0 + r0, M - 1);
+  const C2<T>* a1 = A + min(m0 + r1, M - 1);
+  const bool full = m0 + r1 < M;
+  const C2<T>* b[NS];
+#pragma unroll
+  for (int n = 0; n < NS; ++n) b[n] = B + (int64_t)min(n, N - 1) * ldb;
+#pragma unroll 4
+  for (int k = kbeg; k < kend; ++k) {
+    C2<T> av[2];
+    if constexpr (V == 2) {
+      load_run<T, 2>(av, a0 + (int64_t)k * lda, full);
+    } else {
+      av[0] = a0[(int64_t)k * lda];
+      av[1] = a1[(int64_t)k * lda];
     }
-    __syncthreads();
-    if (m < M) {
-      const int kn = min(kSkinnyChunkN, K - k0);
-#pragma unroll 8
-      for (int kk = 0; kk < kn; ++kk) {
-        const C2<T> a = arow[(int64_t)(k0 + kk) * lda];
 #pragma unroll
-        for (int n = 0; n < NS; ++n) {
-          const C2<T> b = bs[kk][n];
-          acc[n].re = fma(a.re, b.re, acc[n].re);
-          acc[n].re = fma(-a.im, b.im, acc[n].re);
-          acc[n].im = fma(a.re, b.im, acc[n].im);
-          acc[n].im = fma(a.im, b.re, acc[n].im);
-        }
+    for (int n = 0; n < NS; ++n) {
+      const C2<T> bv = b[n][k];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        acc[r][n].re = fma(av[r].re, bv.re, acc[r][n].re);
+        acc[r][n].re = fma(-av[r].im, bv.im, acc[r][n].re);
+        acc[r][n].im = fma(av[r].re, bv.im, acc[r][n].im);
+        acc[r][n].im = fma(av[r].im, bv.re, acc[r][n].im);
       }
     }
   }
-  if (m >= M) return;
   const bool use_beta = beta.re != T(0) || beta.im != T(0);
 #pragma unroll
-  for (int n = 0; n < NS; ++n) {
-    if (n >= N) break;
-    C2<T>* c = C + m + (int64_t)n * ldc;
-    C2<T> v = qeb::cmul(alpha, acc[n]);
-    if (use_beta) v = v + qeb::cmul(beta, *c);
-    *c = v;
+  for (int n0 = 0; n0 < NS; n0 += kStep) {
+    if (n0 > 0) __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kStep; ++j)
+      if (n0 + j < NS) {
+        part[warp][j][r0] = acc[0][n0 + j];
+        part[warp][j][r1] = acc[1][n0 + j];
+      }
+    __syncthreads();
+    const int j = threadIdx.x / kSkinnyRows, r = threadIdx.x % kSkinnyRows;
+    const int m = m0 + r, n = n0 + j;
+    if (n < NS && n < N && m < M) {
+      C2<T> sum = part[0][j][r];
+#pragma unroll
+      for (int w = 1; w < kSkinnyWarps; ++w) sum = sum + part[w][j][r];
+      C2<T>* c = C + m + (int64_t)n * ldc;
+      C2<T> v = qeb::cmul(alpha, sum);
+      if (use_beta) v = v + qeb::cmul(beta, *c);
+      *c = v;
+    }
   }
 }
+static_assert(kSkinnyThreads == 4 * kSkinnyRows, "one output per thread and reduction step");
 
 int g_sm_count = 0;
 
@@ -547,11 +602,26 @@ int mma_splits(int M, int N, int K) {
   return best;
 }
 
+// Compiled widths of the narrow side.
+constexpr int kSkinnyWidths[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16};
+
+int skinny_width(int n) {
+  for (int w : kSkinnyWidths)
+    if (n <= w) return w;
+  return kSkinnyMax;
+}
+
 // Skinny OP_C plan: the narrow side (N, else M when N is wide), the large
-// side Mb and the number of K slices (about four waves, each >= 1024 deep).
+// side mb, the number of K slices (two waves of two blocks per SM, each slice
+// at least 1024 deep) and whether the warps of a block split K between them
+// (wk: when the blocks would not fill the GPU otherwise).
 struct SkinnyC {
   bool use = false, swapped = false;
-  int mb = 0, ns = 0, splits = 1;
+  int mb = 0, ns = 0, splits = 1, wk = 1;
+  int groups() const {  // blocks along the large side
+    const int per = skinny_cols(skinny_width(ns)) * (kSkinnyWarps / wk);
+    return (mb + per - 1) / per;
+  }
 };
 
 SkinnyC skinny_c_plan(int M, int N, int K) {
@@ -563,23 +633,64 @@ SkinnyC skinny_c_plan(int M, int N, int K) {
   } else {
     return p;
   }
-  const int groups = (p.mb + kSkinnyColumns - 1) / kSkinnyColumns;
-  int want = (4 * sm_count() + groups - 1) / groups;
-  int by_depth = K / 1024;
-  if (by_depth < 1) by_depth = 1;
-  int s = want < by_depth ? want : by_depth;
-  if (s > 64) s = 64;
-  p.splits = s < 1 ? 1 : s;
+  const int by_depth = K / 1024 < 1 ? 1 : K / 1024;
+  if ((int64_t)p.groups() * by_depth < 2 * sm_count()) p.wk = kSkinnyWarps;
+  const int fill = 4 * sm_count() / p.groups();
+  // a split product needs a second launch: not for the depth one block
+  // covers in a few loads per lane
+  const int deep = p.wk > 1 ? K / 4096 : by_depth;
+  p.splits = fill < deep ? fill : deep;
+  if (p.splits > 64) p.splits = 64;
+  if (p.splits < 1) p.splits = 1;
   return p;
 }
 
 template <typename T, int NS>
-void launch_skinny_c(const SkinnyC& p, int K, int krange, const C2<T>* X, int64_t ldx,
+void launch_skinny_c(const SkinnyC& p, bool wide, int K, int krange, const C2<T>* X, int64_t ldx,
                      const C2<T>* Y, int64_t ldy, C2<T> al, C2<T> be, C2<T>* C, int64_t ldc,
                      C2<T>* partials, cudaStream_t stream) {
-  const dim3 grid((p.mb + kSkinnyColumns - 1) / kSkinnyColumns, p.splits);
-  skinny_c_kernel<T, NS><<<grid, kSkinnyThreads, 0, stream>>>(
-      p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, p.swapped ? 1 : 0, partials);
+  const dim3 grid(p.groups(), p.splits);
+  constexpr int V = sizeof(T) == 4 ? 2 : 1;
+  const int sw = p.swapped ? 1 : 0;
+  if (p.wk > 1) {
+    if (wide)
+      skinny_c_kernel<T, NS, V, kSkinnyWarps><<<grid, kSkinnyThreads, 0, stream>>>(
+          p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
+    else
+      skinny_c_kernel<T, NS, 1, kSkinnyWarps><<<grid, kSkinnyThreads, 0, stream>>>(
+          p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
+  } else if (wide) {
+    skinny_c_kernel<T, NS, V, 1><<<grid, kSkinnyThreads, 0, stream>>>(
+        p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
+  } else {
+    skinny_c_kernel<T, NS, 1, 1><<<grid, kSkinnyThreads, 0, stream>>>(
+        p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
+  }
+}
+
+// Whether complex64 columns start on 16-byte boundaries (two values a load);
+// complex128 values are 16-byte loads in any case.
+template <typename T>
+bool wide_loads(const C2<T>* p, int64_t ld) {
+  return sizeof(T) == 8 || (reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 2 == 0);
+}
+
+// Calls fn(integral_constant<width>) for the compiled width of n.
+template <class Fn>
+void with_width(int n, Fn&& fn) {
+  switch (skinny_width(n)) {
+    case 1: fn(std::integral_constant<int, 1>{}); break;
+    case 2: fn(std::integral_constant<int, 2>{}); break;
+    case 3: fn(std::integral_constant<int, 3>{}); break;
+    case 4: fn(std::integral_constant<int, 4>{}); break;
+    case 5: fn(std::integral_constant<int, 5>{}); break;
+    case 6: fn(std::integral_constant<int, 6>{}); break;
+    case 7: fn(std::integral_constant<int, 7>{}); break;
+    case 8: fn(std::integral_constant<int, 8>{}); break;
+    case 10: fn(std::integral_constant<int, 10>{}); break;
+    case 12: fn(std::integral_constant<int, 12>{}); break;
+    default: fn(std::integral_constant<int, 16>{}); break;
+  }
 }
 
 template <typename T>
@@ -592,22 +703,20 @@ int gemm_skinny_c(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, co
     const int64_t fit = (scratch == nullptr) ? 0 : scratch_bytes / slice_bytes;
     if (fit < p.splits) p.splits = (int)(fit < 1 ? 1 : fit);
   }
+  constexpr int kChunk = 64;  // slices start on whole 16-byte loads of a warp
   int krange = (K + p.splits - 1) / p.splits;
-  krange = (krange + kSkinnyChunkC - 1) / kSkinnyChunkC * kSkinnyChunkC;
-  if (krange < 1) krange = kSkinnyChunkC;
-  p.splits = K > 0 ? (K + krange - 1) / krange : 1;
+  krange = (krange + kChunk - 1) / kChunk * kChunk;
+  p.splits = (K + krange - 1) / krange;
   // large operand X and narrow operand Y of D = X^H Y
   const C2<T>* X = p.swapped ? B : A;
   const C2<T>* Y = p.swapped ? A : B;
   const int64_t ldx = p.swapped ? ldb : lda, ldy = p.swapped ? lda : ldb;
+  const bool wide = wide_loads(X, ldx) && wide_loads(Y, ldy);
   C2<T>* partials = p.splits > 1 ? static_cast<C2<T>*>(scratch) : nullptr;
-  const int width = skinny_width(p.ns);
-  if (width == 4)
-    launch_skinny_c<T, 4>(p, K, krange, X, ldx, Y, ldy, al, be, C, ldc, partials, stream);
-  else if (width == 8)
-    launch_skinny_c<T, 8>(p, K, krange, X, ldx, Y, ldy, al, be, C, ldc, partials, stream);
-  else
-    launch_skinny_c<T, 16>(p, K, krange, X, ldx, Y, ldy, al, be, C, ldc, partials, stream);
+  with_width(p.ns, [&](auto w) {
+    launch_skinny_c<T, decltype(w)::value>(p, wide, K, krange, X, ldx, Y, ldy, al, be, C, ldc,
+                                           partials, stream);
+  });
   qeb::count_launches(p.splits > 1 ? 2 : 1);
   if (p.splits > 1) {
     const int64_t total = (int64_t)p.mb * p.ns;
@@ -622,14 +731,20 @@ int gemm_skinny_c(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, co
 template <typename T>
 int gemm_skinny_n(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, const C2<T>* B,
                   int64_t ldb, C2<T> be, C2<T>* C, int64_t ldc, cudaStream_t stream) {
-  const dim3 grid((M + kSkinnyThreads - 1) / kSkinnyThreads);
-  const int width = skinny_width(N);
-  if (width == 4)
-    skinny_n_kernel<T, 4><<<grid, kSkinnyThreads, 0, stream>>>(M, N, K, al, A, lda, B, ldb, be, C, ldc);
-  else if (width == 8)
-    skinny_n_kernel<T, 8><<<grid, kSkinnyThreads, 0, stream>>>(M, N, K, al, A, lda, B, ldb, be, C, ldc);
-  else
-    skinny_n_kernel<T, 16><<<grid, kSkinnyThreads, 0, stream>>>(M, N, K, al, A, lda, B, ldb, be, C, ldc);
+  const dim3 grid((M + kSkinnyRows - 1) / kSkinnyRows);
+  const bool wide = sizeof(T) == 4 && wide_loads(A, lda);
+  with_width(N, [&](auto w) {
+    constexpr int NS = decltype(w)::value;
+    if constexpr (sizeof(T) == 4) {
+      if (wide) {
+        skinny_n_kernel<T, NS, 2><<<grid, kSkinnyThreads, 0, stream>>>(M, N, K, al, A, lda, B,
+                                                                       ldb, be, C, ldc);
+        return;
+      }
+    }
+    skinny_n_kernel<T, NS, 1><<<grid, kSkinnyThreads, 0, stream>>>(M, N, K, al, A, lda, B, ldb,
+                                                                   be, C, ldc);
+  });
   qeb::count_launches(1);
   return qeb::cuda_status(cudaGetLastError(), "zgemm skinny launch");
 }
