@@ -315,6 +315,27 @@ int qeb_subtract_band_energies(int precision, int64_t rows, int64_t cols, void* 
                                int64_t ldr, const void* v, int64_t ldv, const double* energies,
                                void* stream);
 
+/* Lowest `roots` pairs of the Hermitian pencil H c = e S c, n <= 32
+ * (qeb_small_eigh_max), in one launch: H and S row-major complex128 (of S the
+ * lower triangle is read), `values` roots + 1 doubles on the device, vectors
+ * column-major n x roots, S-orthonormal.  values[roots]: 0, or k > 0 when the
+ * Cholesky factorisation of S failed at row k, or -1 when the rotations did not
+ * converge; values and vectors are then undefined.  Replaces LAPACK zhegv
+ * (qepy_pw/diagonalization.py:83-110) for small subspaces. */
+int qeb_small_eigh_max(void);
+int qeb_small_generalized_eigh(int n, int roots, const void* h, int64_t ldh, const void* s,
+                               int64_t lds, double* values, void* vectors, int64_t ldv,
+                               void* stream);
+
+/* Rows [first, active) of the reduced matrices (row-major complex128, leading
+ * dimension ld) from new^H [H V, V] (column-major, `precision`), their conjugates
+ * in the columns above them, the new diagonal block averaged with its conjugate
+ * transpose (qepy_pw/diagonalization.py:658-695).  lam (or null): h_rows += s_rows
+ * lam on the first nlam columns beforehand. */
+int qeb_update_reduced(int precision, int first, int active, const void* h_rows, int64_t ldh,
+                       const void* s_rows, int64_t lds, const double* lam, int nlam,
+                       void* projected, void* overlap, int64_t ld, void* stream);
+
 /* diag[g] += multiplicity * Re sum_i coupled[g,i] conj(beta[g,i]) (coupled = beta D)
  * — accumulate_projector_diagonal (qepy_pw/_native_fft.pyx:734-779) */
 int qeb_accumulate_projector_diagonal(int precision, int64_t rows, int64_t channels,

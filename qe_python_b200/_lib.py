@@ -70,6 +70,9 @@ SIGNATURES: list[tuple[str, object, list]] = [
     ("qeb_column_inner_products", _I, [_I, _L, _L, _P, _L, _P, _L, _P, _P]),
     ("qeb_precondition", _I, [_I, _L, _L, _P, _L, _P, _P, _P, _L, _P]),
     ("qeb_normalize_columns", _I, [_I, _L, _L, _P, _L, _P, _P, _P, _L, _P]),
+    ("qeb_small_eigh_max", _I, []),
+    ("qeb_small_generalized_eigh", _I, [_I, _I, _P, _L, _P, _L, _P, _P, _L, _P]),
+    ("qeb_update_reduced", _I, [_I, _I, _I, _P, _L, _P, _L, _P, _I, _P, _P, _L, _P]),
     ("qeb_subtract_band_energies", _I, [_I, _L, _L, _P, _L, _P, _L, _P, _P]),
     ("qeb_accumulate_projector_diagonal", _I, [_I, _L, _L, _P, _L, _P, _L, _D, _P, _P]),
 ]

@@ -990,16 +990,9 @@ def davidson_steps(diagonal, number_of_roots: int, *, initial_vectors=None,
         """New rows/columns of V^H H V and V^H V (:658-695)."""
         with _timer(timers, "cegterg:over"):
             new = basis_storage[:, first_new:active]
-            h_rows = K.gemm(K.OP_C, new, applied_storage[:, :active]).to(torch.complex128)
-            s_rows = K.gemm(K.OP_C, new, basis_storage[:, :active]).to(torch.complex128)
-            projected[first_new:active, :active] = h_rows
-            overlap[first_new:active, :active] = s_rows
-            if first_new:
-                projected[:first_new, first_new:active] = h_rows[:, :first_new].conj().T
-                overlap[:first_new, first_new:active] = s_rows[:, :first_new].conj().T
-            block = slice(first_new, active)
-            projected[block, block] = _hermitize(projected[block, block])
-            overlap[block, block] = _hermitize(overlap[block, block])
+            h_rows = K.gemm(K.OP_C, new, applied_storage[:, :active])
+            s_rows = K.gemm(K.OP_C, new, basis_storage[:, :active])
+            K.update_reduced(projected, overlap, first_new, h_rows, s_rows)
 
     nroot = number_of_roots  # roots of the reduced problem (fewer once some are locked)
     root_ids = np.arange(number_of_roots)  # their indices among all roots
@@ -1015,7 +1008,7 @@ def davidson_steps(diagonal, number_of_roots: int, *, initial_vectors=None,
             yield OVERLAP
         with _timer(timers, "cdiaghg"):
             roots, coefficients = solver.result()
-        return roots.cpu().numpy(), roots, coefficients
+        return solver.host_values(), roots, coefficients
 
     def ritz_columns(coefficients, roots, columns=None):
         """Ritz vectors V c and residuals HV c - e V c (:709-724) of the
@@ -1350,16 +1343,9 @@ def refined_davidson_steps(diagonal, number_of_roots: int, *, initial_vectors,
     def update_projected(first_new: int, active: int, lam_dev) -> None:
         with _timer(timers, "cegterg:over"):
             new = basis32[:, first_new:active]
-            h_rows = K.gemm(K.OP_C, new, applied32[:, :active]).to(torch.complex128)
-            s_rows = K.gemm(K.OP_C, new, basis32[:, :active]).to(torch.complex128)
-            h_rows[:, :n] += s_rows[:, :n] * lam_dev.to(torch.complex128)[None, :]
-            projected[first_new:active, :active] = h_rows
-            overlap[first_new:active, :active] = s_rows
-            projected[:first_new, first_new:active] = h_rows[:, :first_new].conj().T
-            overlap[:first_new, first_new:active] = s_rows[:, :first_new].conj().T
-            block = slice(first_new, active)
-            projected[block, block] = _hermitize(projected[block, block])
-            overlap[block, block] = _hermitize(overlap[block, block])
+            h_rows = K.gemm(K.OP_C, new, applied32[:, :active])
+            s_rows = K.gemm(K.OP_C, new, basis32[:, :active])
+            K.update_reduced(projected, overlap, first_new, h_rows, s_rows, lam_dev)
 
     def composite_residuals(coefficients, roots, lam_dev, active):
         """FP32 residuals H V c - e V c of the selected roots."""

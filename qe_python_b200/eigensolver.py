@@ -14,7 +14,8 @@ Several k points' solves, each a chain of small latency-bound kernels, then
 run side by side on the GPU; the host reads the error codes when it reads
 the eigenvalues.
 
-``ReducedSolve.launch`` enqueues a solve on a stream and returns at once;
+Small subspaces (SMALL_LIMIT) take one kernel of libqeb200.so instead of that
+chain.  ``ReducedSolve.launch`` enqueues a solve on a stream and returns at once;
 ``ReducedSolve.result`` makes the current stream wait for it and returns the
 lowest ``roots`` pairs, or falls back to the canonical orthogonalisation of
 the overlap when S was not numerically positive definite.
@@ -25,11 +26,17 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+from contextlib import nullcontext
 
 import torch
 
+from . import _lib
+
 _P, _I = ctypes.c_void_p, ctypes.c_int
 _MODE_VECTOR, _FILL_LOWER = 1, 0
+
+# Columns up to which the one-launch solver is the faster one.
+SMALL_LIMIT = 32
 
 _lock = threading.Lock()
 _state: dict = {}
@@ -109,15 +116,48 @@ def zheevd_async(matrix: torch.Tensor, stream: torch.cuda.Stream):
 
 
 class ReducedSolve:
-    """One asynchronous solve of H c = e S c for the lowest ``roots`` pairs."""
+    """One asynchronous solve of H c = e S c for the lowest ``roots`` pairs.
+
+    Subspaces of up to SMALL_LIMIT columns go to the one-launch kernel
+    (qeb_small_generalized_eigh), larger ones, and those whose rotations did
+    not converge, to the Cholesky reduction and zheevd."""
 
     def __init__(self, stream: torch.cuda.Stream) -> None:
         self.stream = stream
         self._pending = None
+        self._host = None  # the last result's values on the host, when already there
+        self._values = None
 
     def launch(self, h: torch.Tensor, s: torch.Tensor, roots: int) -> None:
         """Enqueue the solve of the Hermitian pair (h, s) on the stream after
         the work the current stream has enqueued so far."""
+        n = h.shape[0]
+        if n <= SMALL_LIMIT and 1 <= roots <= n and all(
+                m.dtype == torch.complex128 and m.is_cuda and m.stride(1) == 1 and m.stride(0) >= n
+                for m in (h, s)):
+            self._launch_small(h, s, roots)
+        else:
+            self._launch_library(h, s, roots)
+
+    def _launch_small(self, h: torch.Tensor, s: torch.Tensor, roots: int) -> None:
+        n = h.shape[0]
+        current = torch.cuda.current_stream(h.device)
+        same = self.stream == current
+        if not same:
+            self.stream.wait_stream(current)
+        with nullcontext() if same else torch.cuda.stream(self.stream):
+            values = torch.empty(roots + 1, dtype=torch.float64, device=h.device)
+            vectors = torch.empty((roots, n), dtype=torch.complex128, device=h.device).T
+            _lib.check("qeb_small_generalized_eigh", _lib.load().qeb_small_generalized_eigh(
+                n, roots, h.data_ptr(), h.stride(0), s.data_ptr(), s.stride(0),
+                values.data_ptr(), vectors.data_ptr(), n, int(self.stream.cuda_stream)))
+            done = None
+            if not same:
+                done = torch.cuda.Event()
+                done.record(self.stream)
+        self._pending = ("small", h, s, roots, values, vectors, done, current)
+
+    def _launch_library(self, h: torch.Tensor, s: torch.Tensor, roots: int) -> None:
         from .diagonalization import _hermitize
 
         current = torch.cuda.current_stream(h.device)
@@ -135,14 +175,49 @@ class ReducedSolve:
             values = values[:roots]
             done = torch.cuda.Event()
             done.record(self.stream)
-        self._pending = (h, s, roots, values, vectors, chol_info, eig_info, done, current)
+        self._pending = ("library", h, s, roots, values, vectors, chol_info, eig_info, done,
+                         current)
 
     def result(self):
         """(values, vectors) of the launched solve, on the current stream."""
+        self._host = None
+        if self._pending[0] == "small":
+            solved = self._result_small()
+            if solved is None:  # not converged: the library route
+                _, h, s, roots, *_ = self._pending
+                self._launch_library(h, s, roots)
+                solved = self._result_library()
+        else:
+            solved = self._result_library()
+        self._pending = None
+        self._values = solved[0]
+        return solved
+
+    def host_values(self):
+        """The values of the last ``result`` as a NumPy array."""
+        return self._values.cpu().numpy() if self._host is None else self._host
+
+    def _result_small(self):
         from .diagonalization import _canonical_generalized_eigh
 
-        h, s, roots, values, vectors, chol_info, eig_info, done, current = self._pending
-        self._pending = None
+        _, h, s, roots, values, vectors, done, current = self._pending
+        if done is not None:
+            current.wait_event(done)
+            for tensor in (h, s, values, vectors):
+                tensor.record_stream(current)
+        host = values.cpu().numpy()
+        status = int(host[roots])
+        if status > 0:
+            return _canonical_generalized_eigh(h, s, roots)
+        if status < 0:
+            return None
+        self._host = host[:roots]
+        return values[:roots], vectors
+
+    def _result_library(self):
+        from .diagonalization import _canonical_generalized_eigh
+
+        _, h, s, roots, values, vectors, chol_info, eig_info, done, current = self._pending
         current.wait_event(done)
         for tensor in (h, s, values, vectors, chol_info, eig_info):
             tensor.record_stream(current)

@@ -467,3 +467,26 @@ def accumulate_projector_diagonal(diagonal: torch.Tensor, coupled: torch.Tensor,
         leading_dimension(coupled), beta.data_ptr(), leading_dimension(beta),
         float(multiplicity), diagonal.data_ptr(), stream_handle()))
     return diagonal
+
+
+def update_reduced(projected: torch.Tensor, overlap: torch.Tensor, first: int,
+                   h_rows: torch.Tensor, s_rows: torch.Tensor,
+                   lam: torch.Tensor | None = None) -> None:
+    """New rows [first, first + m) of the row-major reduced matrices from
+    h_rows, s_rows = new^H [H V, V] (m x active), with the Hermitian
+    counterparts; ``lam`` adds s_rows lam to h_rows on its columns."""
+    _check_matrix("h_rows", h_rows)
+    _check_matrix("s_rows", s_rows)
+    rows, active = h_rows.shape
+    if s_rows.shape != h_rows.shape or s_rows.dtype != h_rows.dtype or active != first + rows:
+        raise ValueError("reduced rows disagree")
+    for m in (projected, overlap):
+        if m.dtype != torch.complex128 or m.stride(1) != 1 or m.shape[0] < active or \
+                m.shape[1] < active or m.stride(0) != projected.stride(0):
+            raise ValueError("the reduced matrices must be row-major complex128 of one size")
+    values = None if lam is None else lam.to(dtype=torch.float64).contiguous()
+    _lib.check("qeb_update_reduced", _lib.load().qeb_update_reduced(
+        _precision(h_rows), first, active, h_rows.data_ptr(), leading_dimension(h_rows),
+        s_rows.data_ptr(), leading_dimension(s_rows), 0 if values is None else values.data_ptr(),
+        0 if values is None else values.numel(), projected.data_ptr(), overlap.data_ptr(),
+        projected.stride(0), stream_handle()))
