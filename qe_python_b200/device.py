@@ -31,11 +31,11 @@ def require_cuda() -> torch.device:
 
 
 def stream_handle(stream: torch.cuda.Stream | None = None) -> int:
-    # current_stream() without a device asks torch for the available device
-    # type, a CUDA device-count query (~0.5 ms) on every call; with the
-    # current device index it does not
+    # the raw handle of the current stream: building a torch.cuda.Stream for
+    # every launch took several microseconds, and without a device index a
+    # device-count query (~0.5 ms) besides
     if stream is None:
-        stream = torch.cuda.current_stream(torch.cuda.current_device())
+        return int(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     return int(stream.cuda_stream)
 
 
@@ -67,8 +67,9 @@ def empty_f(rows: int, cols: int, dtype, device=None, ld: int | None = None) -> 
     """Uninitialised column-major (rows, cols) tensor."""
     device = device if device is not None else require_cuda()
     ld = aligned_ld(rows) if ld is None else ld
-    storage = torch.empty((cols, ld), dtype=dtype, device=device)
-    return storage.T[:rows]
+    if ld == rows:
+        return torch.empty_strided((rows, cols), (1, rows), dtype=dtype, device=device)
+    return torch.empty((cols, ld), dtype=dtype, device=device).as_strided((rows, cols), (1, ld))
 
 
 def zeros_f(rows: int, cols: int, dtype, device=None) -> torch.Tensor:

@@ -210,6 +210,15 @@ class _DeviceProjectors:
                                             float(multiplicity))
 
 
+# Projector multiply-adds from which H|psi> runs them on a side stream beside
+# the FFT passes; below, forking and joining the stream costs the host more
+# than the overlap gains.  Measured, side stream against one stream: 8 bands of
+# 579 plane waves, 8 channels (4e4) 103 and 59 us; 24 bands of the 8-atom cell
+# (2e6) 98 and 65; 4 bands of the 64-atom cell (2e7) FP64 105 and 134; 37 bands
+# of a slab (6e7) 161 and 179.
+OVERLAP_MIN_MACS = 1 << 24
+
+
 class PlaneWaveHamiltonian:
     """H = T + V_loc + sum |beta> D <beta| applied on the GPU.
 
@@ -346,7 +355,9 @@ class PlaneWaveHamiltonian:
         if target is None:
             target = empty_f(vectors.shape[0], vectors.shape[1], self.dtype, self.device)
         nonlocal_part = self.projectors.beta is not None and vectors.shape[1] > 0
-        if nonlocal_part and self.timers is None:
+        overlapped = nonlocal_part and self.timers is None and (
+            vectors.numel() * self.projectors.channels >= OVERLAP_MIN_MACS)
+        if overlapped:
             # beta^H psi and D becp need only psi: they run on a side stream
             # while the FFT passes write the local part into target, and the
             # projector add joins after both

@@ -8,6 +8,7 @@ the current torch stream.  Matrices are column-major torch CUDA tensors
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import numpy as np
@@ -23,6 +24,12 @@ OP_C = 1
 _PREC = {torch.complex128: _lib.QEB_F64, torch.complex64: _lib.QEB_F32}
 
 
+@functools.lru_cache(maxsize=64)
+def _scalar(value: complex):
+    """A complex scalar as the (re, im) doubles that the library reads."""
+    return (ctypes.c_double * 2)(value.real, value.imag)
+
+
 class _Scratch:
     """Grow-only device scratch for split-K partial tiles, one buffer per
     (device, stream): products issued on different streams never share it.
@@ -35,7 +42,8 @@ class _Scratch:
         self._retired: list[torch.Tensor] = []
 
     def get(self, nbytes: int, device: torch.device) -> torch.Tensor:
-        key = (device, torch.cuda.current_stream(device).cuda_stream)
+        key = (device, torch._C._cuda_getCurrentRawStream(
+            torch._C._cuda_getDevice() if device.index is None else device.index))
         current = self._buffers.get(key)
         if current is None or current.numel() < nbytes:
             size = max(int(nbytes), 256)
@@ -123,8 +131,7 @@ def gemm(op_a: int, a: torch.Tensor, b: torch.Tensor, c: torch.Tensor | None = N
     if m == 0 or n == 0:
         return c
     lib = _lib.load()
-    al = (ctypes.c_double * 2)(complex(alpha).real, complex(alpha).imag)
-    be = (ctypes.c_double * 2)(complex(beta).real, complex(beta).imag)
+    al, be = _scalar(complex(alpha)), _scalar(complex(beta))
     need = int(lib.qeb_zgemm_scratch_bytes(op_a, m, n, k, prec))
     scratch = _SCRATCH.get(need, a.device) if need > 0 else None
     fn = lib.qeb_zgemm if prec == _lib.QEB_F64 else lib.qeb_cgemm
@@ -239,8 +246,7 @@ def tf32_gemm(a: PackedOperand, b0: PackedOperand, b1: PackedOperand, c: torch.T
     if m == 0 or n == 0:
         return c
     lib = _lib.load()
-    al = (ctypes.c_double * 2)(complex(alpha).real, complex(alpha).imag)
-    be = (ctypes.c_double * 2)(complex(beta).real, complex(beta).imag)
+    al, be = _scalar(complex(alpha)), _scalar(complex(beta))
     need = int(lib.qeb_tf32_gemm_scratch_bytes(m, n, a.kp))
     scratch = _SCRATCH.get(need, c.device) if need > 0 else None
     _lib.check("qeb_tf32_gemm", lib.qeb_tf32_gemm(
@@ -328,8 +334,7 @@ def cgemm_tf32x3(op_a: int, a: torch.Tensor, b: torch.Tensor, c: torch.Tensor | 
 
 
 def _cgemm_tf32x3_launch(lib, op_a, m, n, k, alpha, a, lda, b, ldb, beta, c, splits):
-    al = (ctypes.c_double * 2)(complex(alpha).real, complex(alpha).imag)
-    be = (ctypes.c_double * 2)(complex(beta).real, complex(beta).imag)
+    al, be = _scalar(complex(alpha)), _scalar(complex(beta))
     if splits and splits > 1:
         need = int(splits) * m * n * 8
     else:

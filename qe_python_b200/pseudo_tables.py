@@ -185,12 +185,18 @@ class SpeciesTables:
         size = int(np.floor(qmax / DQ + 4.0 + 0.5))
         q = np.arange(size) * DQ
         table = np.empty((size, len(p.betas)))
+        # rows are independent: a k point that reaches a little further than
+        # the ones before it adds rows (ten k points made the whole table
+        # four times over)
+        done = 0 if self._beta is None else len(self._beta)
+        if done:
+            table[:done] = self._beta
         pref = 4.0 * np.pi / np.sqrt(self.volume)
         for column, (rbeta, l, cutoff) in enumerate(zip(p.betas, p.angular_momenta, p.cutoff_indices)):
             count = min(cutoff, len(p.r), len(rbeta))
             r = p.r[:count]
             radial = rbeta[:count] * r
-            for b in range(0, size, 128):
+            for b in range(done, size, 128):
                 bessel = spherical_jn(l, np.multiply.outer(q[b:b + 128], r)) * radial[None, :]
                 table[b:b + 128, column] = pref * qe_simpson(bessel, p.rab[:count])
         self._beta, self._beta_qmax = table, qmax
