@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, int 
 // of 12 (4 mod 8: the 2 rows x 4 k of a load phase cover all banks), the
 // M-contiguous A of op N is rows of BM values at a stride of BM + 2 (2 mod 8).
 // Measured against the SIMT kernel: the 23 847 x 184 x 184 rotation 0.373 ->
-// 0.250 ms (25.8 TFLOP/s), H|psi> of 256 bands on 64^3 1.895 -> 1.343 ms.
+// 0.219 ms (29.5 TFLOP/s).
 constexpr int kMmaK = 8, kMmaStages = 4, kMmaThreads = 128, kMmaStride = kMmaK + 4;
 
 template <int BMT, int BNT, bool CONJ_A>
@@ -366,6 +366,38 @@ __device__ __forceinline__ void load_run(C2<T> (&v)[V], const C2<T>* __restrict_
   }
 }
 
+// Asynchronous copy of a run of V values (`valid` of them, the rest zero) to
+// shared memory, and its reading.
+template <typename T, int V>
+__device__ __forceinline__ void copy_run(C2<T>* dst, const C2<T>* __restrict__ src, int valid) {
+  constexpr int bytes = (int)sizeof(C2<T>) * V;
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int size = (int)sizeof(C2<T>) * valid;
+  if constexpr (bytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(size)
+                 : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(size)
+                 : "memory");
+}
+template <typename T, int V>
+__device__ __forceinline__ void read_run(C2<T> (&v)[V], const C2<T>* src) {
+  if constexpr (V == 2) {
+    const float4 w = *reinterpret_cast<const float4*>(src);
+    v[0] = qeb::mk<T>(w.x, w.y);
+    v[1] = qeb::mk<T>(w.z, w.w);
+  } else {
+    v[0] = src[0];
+  }
+}
+
+constexpr int kSkinnyRing = 3;  // steps in the ring of skinny_c_kernel
+
+template <typename T, int NS, int V>
+constexpr size_t skinny_c_smem() {
+  return sizeof(C2<T>) * V * (size_t)kSkinnyRing * (skinny_cols(NS) + NS) * kSkinnyThreads;
+}
+
 // D[mb, ns] = sum_k conj(X[k, mb]) Y[k, ns] over this block's K range.  A warp
 // owns MC columns of X and reads them with MC + NS loads per 4 MC NS
 // multiply-adds, lanes along k (one column per warp with Y staged in shared
@@ -397,26 +429,47 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_c_kernel(
   for (int i = 0; i < MC; ++i)
 #pragma unroll
     for (int n = 0; n < NS; ++n) acc[i][n] = qeb::mk<T>(0, 0);
-  if (m0 < Mb) {
-    for (int k = kbeg + ((warp % WK) * 32 + lane) * V; k < kend; k += WK * 32 * V) {
-      const bool full = k + V <= kend;
-      C2<T> xv[MC][V], yv[NS][V];
+  // a ring of runs in shared memory, private to the thread: copies of the next
+  // kRing - 1 steps are in flight while one is multiplied, without a barrier
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C2<T>* ring = reinterpret_cast<C2<T>*>(smem_raw) + (size_t)threadIdx.x * V;
+  constexpr int kSlot = kSkinnyThreads * V, kStep = WK * 32 * V;
+  const int first = kbeg + ((warp % WK) * 32 + lane) * V;
+  const int steps = m0 < Mb && first < kend ? (kend - first + kStep - 1) / kStep : 0;
+  auto fetch = [&](int step) {
+    if (step < steps) {
+      const int k = first + step * kStep;
+      const int valid = min(V, kend - k);
+      C2<T>* slot = ring + (size_t)(step % kSkinnyRing) * (MC + NS) * kSlot;
 #pragma unroll
-      for (int i = 0; i < MC; ++i) load_run<T, V>(xv[i], x[i] + k, full);
+      for (int i = 0; i < MC; ++i) copy_run<T, V>(slot + i * kSlot, x[i] + k, valid);
 #pragma unroll
-      for (int n = 0; n < NS; ++n) load_run<T, V>(yv[n], y[n] + k, full);
-#pragma unroll
-      for (int v = 0; v < V; ++v)
-#pragma unroll
-        for (int i = 0; i < MC; ++i)
-#pragma unroll
-          for (int n = 0; n < NS; ++n) {  // conj(x) * y
-            acc[i][n].re = fma(xv[i][v].re, yv[n][v].re, acc[i][n].re);
-            acc[i][n].re = fma(xv[i][v].im, yv[n][v].im, acc[i][n].re);
-            acc[i][n].im = fma(xv[i][v].re, yv[n][v].im, acc[i][n].im);
-            acc[i][n].im = fma(-xv[i][v].im, yv[n][v].re, acc[i][n].im);
-          }
+      for (int n = 0; n < NS; ++n) copy_run<T, V>(slot + (MC + n) * kSlot, y[n] + k, valid);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int step = 0; step < kSkinnyRing - 1; ++step) fetch(step);
+  for (int step = 0; step < steps; ++step) {
+    fetch(step + kSkinnyRing - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSkinnyRing - 1) : "memory");
+    const C2<T>* slot = ring + (size_t)(step % kSkinnyRing) * (MC + NS) * kSlot;
+    C2<T> xv[MC][V], yv[NS][V];
+#pragma unroll
+    for (int i = 0; i < MC; ++i) read_run<T, V>(xv[i], slot + i * kSlot);
+#pragma unroll
+    for (int n = 0; n < NS; ++n) read_run<T, V>(yv[n], slot + (MC + n) * kSlot);
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int i = 0; i < MC; ++i)
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {  // conj(x) * y
+          acc[i][n].re = fma(xv[i][v].re, yv[n][v].re, acc[i][n].re);
+          acc[i][n].re = fma(xv[i][v].im, yv[n][v].im, acc[i][n].re);
+          acc[i][n].im = fma(xv[i][v].re, yv[n][v].im, acc[i][n].im);
+          acc[i][n].im = fma(-xv[i][v].im, yv[n][v].re, acc[i][n].im);
+        }
   }
   C2<T> mine = qeb::mk<T>(0, 0);  // lane l: entry (l / NS, l % NS), then l + 32, ...
   __shared__ C2<T> part[WK > 1 ? kSkinnyWarps : 1][MC * NS];
@@ -479,7 +532,7 @@ __global__ void skinny_reduce(int Mb, int Ns, int splits, const C2<T>* __restric
 // meet in shared memory four columns at a time.  (One thread per row over the
 // whole of K left 2.1 blocks of 256 rows per SM on the 216-atom cell's
 // projector add, 80 725 x 864 x 5 complex64.)  With the kernel above: H|psi> of 5
-// bands of that cell 0.574 -> 0.409 ms.
+// bands of that cell 0.574 -> 0.347 ms.
 template <typename T, int NS, int V>
 __global__ void __launch_bounds__(kSkinnyThreads) skinny_n_kernel(
     int M, int N, int K, C2<T> alpha, const C2<T>* __restrict__ A, int64_t lda,
@@ -570,35 +623,37 @@ int choose_splits(int M, int N, int K) {
   return s < 1 ? 1 : s;
 }
 
-// Tile of the FP64 tensor kernel: per dimension the edge of 64, 48 or 32 with
-// the least padding (the larger one on a tie: fewer loads per product).
-int mma_edge(int n) {
-  int best = 64, cost = (n + 63) / 64 * 64;
-  for (int e : {48, 32}) {
-    const int c = (n + e - 1) / e * e;
-    if (c < cost) best = e, cost = c;
-  }
-  return best;
-}
-
-// K slices of the FP64 tensor kernel: the blocks of one SM share its FP64
-// pipe, so the time is that of the SM with the most tiles (at kSmRate
-// complex multiply-adds per microsecond), plus writing and reading the
-// partial slices; slices are at least 64 deep.  The rates only weigh the two
+// Tile edges (64, 48 or 32) and K slices of the FP64 tensor kernel.  The blocks
+// of one SM share its FP64 pipe, so the time is that of the SM with the most
+// tiles (at kSmRate complex multiply-adds per microsecond), plus writing and
+// reading the partial slices of a split; slices are at least 64 deep.  Against
+// that, A B runs faster in small tiles, of which more blocks are resident
+// (23 847 x 184 x 184: 32 x 32 243 us, 48 x 48 260; 80 725 x 97 x 300: 32 x 32 804,
+// 64 x 64 957), A^H B a little faster in large ones, which load less per product
+// (512 x 256 x 11 019: 64 x 64 370 us, 32 x 32 385).  The rates only weigh the
 // terms against each other.
-int mma_splits(int M, int N, int K) {
+struct MmaPlan {
+  int bm = 64, bn = 64, splits = 1;
+};
+
+MmaPlan mma_plan(int M, int N, int K, bool split) {
   constexpr double kSmRate = 30.0e3, kSliceBytes = 4.0e6;  // per SM; bytes per us
-  const int bm = mma_edge(M), bn = mma_edge(N);
-  const int64_t tiles = (int64_t)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-  int best = 1;
+  MmaPlan best;
   double best_time = 0.0;
-  for (int s = 1; s <= 64 && (s == 1 || K / s >= 64); ++s) {
-    const int64_t per_sm = (tiles * s + sm_count() - 1) / sm_count();
-    const int depth = ((K + s - 1) / s + kMmaK - 1) / kMmaK * kMmaK;
-    double time = (double)per_sm * depth * bm * bn / kSmRate;
-    if (s > 1) time += 2.0 + 32.0 * s * M * N / kSliceBytes;  // a second launch, slices out and in
-    if (s == 1 || time < 0.98 * best_time) best = s, best_time = time;
-  }
+  for (int bm : {64, 48, 32})
+    for (int bn : {64, 48, 32}) {
+      const int64_t tiles = (int64_t)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+      const double rate = kSmRate * (split ? 1.0 - 0.4 / bm - 0.4 / bn
+                                           : 1.0 - 0.05 * (bm * bn / 1024.0 - 1.0));
+      for (int s = 1; s <= (split ? 64 : 1) && (s == 1 || K / s >= 64); ++s) {
+        const int64_t per_sm = (tiles * s + sm_count() - 1) / sm_count();
+        const int depth = ((K + s - 1) / s + kMmaK - 1) / kMmaK * kMmaK;
+        double time = (double)per_sm * depth * bm * bn / rate;
+        if (s > 1) time += 2.0 + 32.0 * s * M * N / kSliceBytes;  // a second launch, slices
+        if (best_time == 0.0 || time < 0.99 * best_time)
+          best.bm = bm, best.bn = bn, best.splits = s, best_time = time;
+      }
+    }
   return best;
 }
 
@@ -646,26 +701,24 @@ SkinnyC skinny_c_plan(int M, int N, int K) {
 }
 
 template <typename T, int NS>
-void launch_skinny_c(const SkinnyC& p, bool wide, int K, int krange, const C2<T>* X, int64_t ldx,
+int launch_skinny_c(const SkinnyC& p, bool wide, int K, int krange, const C2<T>* X, int64_t ldx,
                      const C2<T>* Y, int64_t ldy, C2<T> al, C2<T> be, C2<T>* C, int64_t ldc,
                      C2<T>* partials, cudaStream_t stream) {
   const dim3 grid(p.groups(), p.splits);
   constexpr int V = sizeof(T) == 4 ? 2 : 1;
   const int sw = p.swapped ? 1 : 0;
-  if (p.wk > 1) {
-    if (wide)
-      skinny_c_kernel<T, NS, V, kSkinnyWarps><<<grid, kSkinnyThreads, 0, stream>>>(
-          p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
-    else
-      skinny_c_kernel<T, NS, 1, kSkinnyWarps><<<grid, kSkinnyThreads, 0, stream>>>(
-          p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
-  } else if (wide) {
-    skinny_c_kernel<T, NS, V, 1><<<grid, kSkinnyThreads, 0, stream>>>(
-        p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
-  } else {
-    skinny_c_kernel<T, NS, 1, 1><<<grid, kSkinnyThreads, 0, stream>>>(
-        p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be, C, ldc, sw, partials);
-  }
+  auto launch = [&](auto* kernel, size_t smem) {
+    const cudaError_t e = qeb::raise_smem_limit(kernel, smem);
+    if (e != cudaSuccess) return qeb::cuda_status(e, "skinny product shared memory");
+    kernel<<<grid, kSkinnyThreads, smem, stream>>>(p.mb, p.ns, K, krange, X, ldx, Y, ldy, al, be,
+                                                   C, ldc, sw, partials);
+    return QEB_OK;
+  };
+  if (p.wk > 1)
+    return wide ? launch(skinny_c_kernel<T, NS, V, kSkinnyWarps>, skinny_c_smem<T, NS, V>())
+                : launch(skinny_c_kernel<T, NS, 1, kSkinnyWarps>, skinny_c_smem<T, NS, 1>());
+  return wide ? launch(skinny_c_kernel<T, NS, V, 1>, skinny_c_smem<T, NS, V>())
+              : launch(skinny_c_kernel<T, NS, 1, 1>, skinny_c_smem<T, NS, 1>());
 }
 
 // Whether complex64 columns start on 16-byte boundaries (two values a load);
@@ -713,10 +766,12 @@ int gemm_skinny_c(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, co
   const int64_t ldx = p.swapped ? ldb : lda, ldy = p.swapped ? lda : ldb;
   const bool wide = wide_loads(X, ldx) && wide_loads(Y, ldy);
   C2<T>* partials = p.splits > 1 ? static_cast<C2<T>*>(scratch) : nullptr;
+  int rc = QEB_OK;
   with_width(p.ns, [&](auto w) {
-    launch_skinny_c<T, decltype(w)::value>(p, wide, K, krange, X, ldx, Y, ldy, al, be, C, ldc,
-                                           partials, stream);
+    rc = launch_skinny_c<T, decltype(w)::value>(p, wide, K, krange, X, ldx, Y, ldy, al, be, C, ldc,
+                                                partials, stream);
   });
+  if (rc) return rc;
   qeb::count_launches(p.splits > 1 ? 2 : 1);
   if (p.splits > 1) {
     const int64_t total = (int64_t)p.mb * p.ns;
@@ -768,8 +823,7 @@ int launch_mma_tile(int M, int N, int K, int kchunk, int splits, double2 al, con
 }
 
 template <class... Args>
-int launch_mma(int opa, int M, int N, Args... args) {
-  const int bm = mma_edge(M), bn = mma_edge(N);
+int launch_mma(int opa, int bm, int bn, int M, int N, Args... args) {
   const bool conj = opa == QEB_OP_C;
 #define QEB_TILE(m, n)                                                              \
   if (bm == m && bn == n)                                                           \
@@ -812,7 +866,8 @@ int gemm(int opa, int M, int N, int K, const double* alpha, const void* A, int64
                             static_cast<const C2<T>*>(B), ldb, be, static_cast<C2<T>*>(C), ldc,
                             stream);
   constexpr bool kMma = sizeof(T) == 8;
-  int splits = (opa == QEB_OP_C) ? (kMma ? mma_splits(M, N, K) : choose_splits(M, N, K)) : 1;
+  const MmaPlan plan = kMma ? mma_plan(M, N, K, opa == QEB_OP_C) : MmaPlan{};
+  int splits = kMma ? plan.splits : (opa == QEB_OP_C ? choose_splits(M, N, K) : 1);
   const int64_t slice_bytes = (int64_t)M * N * (int64_t)sizeof(C2<T>);
   if (splits > 1) {
     const int64_t fit = (scratch == nullptr) ? 0 : scratch_bytes / slice_bytes;
@@ -828,7 +883,7 @@ int gemm(int opa, int M, int N, int K, const double* alpha, const void* A, int64
   if (K == 0) kchunk = 1;
   C2<T>* partials = (splits > 1) ? static_cast<C2<T>*>(scratch) : nullptr;
   if constexpr (kMma) {
-    const int rc = launch_mma(opa, M, N, K, kchunk, splits, make_double2(al.re, al.im),
+    const int rc = launch_mma(opa, plan.bm, plan.bn, M, N, K, kchunk, splits, make_double2(al.re, al.im),
                               static_cast<const double2*>(A), lda,
                               static_cast<const double2*>(B), ldb, make_double2(be.re, be.im),
                               static_cast<double2*>(C), ldc,
@@ -864,7 +919,8 @@ extern "C" int64_t qeb_zgemm_scratch_bytes(int opa, int M, int N, int K, int pre
     const SkinnyC p = skinny_c_plan(M, N, K);
     return p.splits > 1 ? (int64_t)p.splits * p.mb * p.ns * elem : 0;
   }
-  const int splits = precision == QEB_F64 ? mma_splits(M, N, K) : choose_splits(M, N, K);
+  const int splits =
+      precision == QEB_F64 ? mma_plan(M, N, K, true).splits : choose_splits(M, N, K);
   return splits > 1 ? (int64_t)splits * M * N * elem : 0;
 }
 
