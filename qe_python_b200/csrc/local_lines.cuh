@@ -393,6 +393,23 @@ __device__ __forceinline__ void load_twiddles(C2<T>* inverse, C2<T>* fwd,
   }
 }
 
+// The R twiddles of one role (rows of an even number of values: two complex64
+// values a load; a load per value took 1 to 5 % of the plane pass).
+template <typename T, int R>
+__device__ __forceinline__ void load_role(C2<T> (&w)[even(R)], const C2<T>* p) {
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int k = 0; k < even(R); k += 2) {
+      const float4 v = *reinterpret_cast<const float4*>(p + k);
+      w[k] = mk<T>(v.x, v.y);
+      w[k + 1] = mk<T>(v.z, v.w);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < R; ++k) w[k] = p[k];
+  }
+}
+
 // MODE 0: local potential; MODE 1: density accumulation.
 template <typename T, int MODE, class P>
 __device__ __forceinline__ void plane_body(const KDesc<T>& d, const P& g, int nz,
@@ -432,7 +449,8 @@ __device__ __forceinline__ void plane_body(const KDesc<T>& d, const P& g, int nz
       }
       dft<T, R, true, Z>(v);
       C2<T>* o = plane + a * g.stride + j * R;
-      const C2<T>* w = twy_inv + j * even(R);
+      C2<T> w[even(R)];
+      load_role<T, R>(w, twy_inv + j * even(R));
       o[0] = v[0];
 #pragma unroll
       for (int k = 1; k < R; ++k) o[k] = twiddle_conj(v[k], w[k]);
@@ -473,7 +491,8 @@ __device__ __forceinline__ void plane_body(const KDesc<T>& d, const P& g, int nz
         }
         dft<T, R, true, Z>(v);
         C2<T>* o = buf + j * R * g.columns + c;
-        const C2<T>* w = twx_inv + j * even(R);
+        C2<T> w[even(R)];
+        load_role<T, R>(w, twx_inv + j * even(R));
         o[0] = v[0];
 #pragma unroll
         for (int k = 1; k < R; ++k) o[k * g.columns] = twiddle_conj(v[k], w[k]);
@@ -499,7 +518,8 @@ __device__ __forceinline__ void plane_body(const KDesc<T>& d, const P& g, int nz
 #pragma unroll
           for (int q = 0; q < R; ++q) v[q] = scale(v[q], pot[q]);
           dft<T, R, false>(v);
-          const C2<T>* w = twx_fwd + k * even(R);
+          C2<T> w[even(R)];
+          load_role<T, R>(w, twx_fwd + k * even(R));
           p[0] = v[0];
 #pragma unroll
           for (int q = 1; q < R; ++q) p[q * g.x1 * g.columns] = twiddle(v[q], w[q]);
@@ -547,7 +567,8 @@ __device__ __forceinline__ void plane_body(const KDesc<T>& d, const P& g, int nz
 #pragma unroll
         for (int j = 0; j < R; ++j) v[j] = p[j * g.y1];
         dft<T, R, false>(v);
-        const C2<T>* w = twy_fwd + k * even(R);
+        C2<T> w[even(R)];
+        load_role<T, R>(w, twy_fwd + k * even(R));
         p[0] = v[0];
 #pragma unroll
         for (int q = 1; q < R; ++q) p[q * g.y1] = twiddle(v[q], w[q]);
