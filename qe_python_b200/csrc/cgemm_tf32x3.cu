@@ -23,13 +23,14 @@
 // it into FP32 registers with round-to-nearest.  The result is as accurate
 // as an FP32 FMA GEMM.
 //
-// One CTA = 320 threads computes a 128 x 128 output tile over a K range:
+// One CTA = 320 threads computes a 128 x BN output tile (BN = 128, or 64 for
+// narrow products) over a K range:
 //   warp 0 lane 0 : TMA producer, two stages
 //   warp 1 lane 0 : MMA issuer; warp 1 owns the tensor-memory allocation
 //   warps 2-9     : workers: split the next stage, drain the previous
 //                   stage's accumulator into registers, then store C
 // Worker warp w reads tensor-memory lanes 32 (w % 4) .. +31 (its rows) and
-// columns 64 ((w - 2) / 4) .. +63 of Re and of Im.  K is split across CTAs
+// columns BN / 2 ((w - 2) / 4) .. + BN / 2 - 1 of Re and of Im.  K is split across CTAs
 // (grid.z) into caller scratch when the output has few tiles; a second kernel
 // sums the slices in a fixed order.  Every wait is bounded; on timeout the
 // CTA records an error code in the device word read by qeb_tf32_gemm_error
@@ -41,6 +42,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "qeb_common.cuh"
 #include "tcgen05.cuh"
 #include "../../include/qe_b200.h"
@@ -49,9 +52,14 @@ namespace {
 
 using namespace qeb::tc;
 
-constexpr int BM = 128, BN = 128;
+constexpr int BM = 128;
 constexpr int BKF = 32;      // FP32 words along K per stage (16 complex values)
 constexpr int TILE = 16384;  // bytes of one 128-row x 32-word tile
+// Output columns of a tile: 64 for products of at most 64 columns (a block of
+// bands late in a Davidson solve), which would leave half of a 128-column tile
+// to padding: its split, its products and its accumulators (256 x 61 x 23 847
+// A^H B 80 -> 66 us, 23 847 x 61 x 256 A B 92 -> 74 us).
+int tile_columns(int n) { return n <= 64 ? 64 : 128; }
 constexpr int STAGES = 2;
 // Stages ahead whose tiles the producer prefetches into L2, so that the
 // loads of the two-stage ring read L2 rather than HBM.
@@ -59,37 +67,43 @@ constexpr int kPrefetch = 2;
 constexpr int WORKERS = 8;                 // worker warps (2 .. 9)
 constexpr int WORKER_THREADS = 32 * WORKERS;
 constexpr int THREADS = 64 + WORKER_THREADS;
-constexpr int ACC_COLS = 2 * BN;           // Re and Im of one accumulator buffer
-constexpr int TMEM_COLS = 2 * ACC_COLS;    // two buffers
-constexpr uint32_t kIdesc = idesc_tf32(BM, BN);
-// OP_C: Re and Im share A, so one M128 N256 product over [B; B1] (the two
-// K-major tiles adjacent in shared memory, 256 rows at the same 1024-byte
-// group stride) writes the Re and Im columns of an accumulator buffer at
-// once: 12 KB of operands per 128 x 256 x 8 products instead of 16 KB for
-// two N128 ones.
-constexpr uint32_t kIdescReIm = idesc_tf32(BM, 2 * BN);
+template <int BN>
+struct Shape {
+  static constexpr int b_tile = BN * 128;         // bytes of a BN-row x 32-word tile
+  static constexpr int acc_cols = 2 * BN;         // Re and Im of one accumulator buffer
+  static constexpr int tmem_cols = 2 * acc_cols;  // two buffers
+  static constexpr uint32_t idesc = idesc_tf32(BM, BN);
+  // OP_C: Re and Im share A, so one product over [B; B1] (the two K-major
+  // tiles adjacent in shared memory, 2 BN rows at the same 1024-byte group
+  // stride) writes the Re and Im columns of an accumulator buffer at once: for
+  // BN = 128, 12 KB of operands per 128 x 256 x 8 products instead of 16 KB for
+  // two N128 ones.
+  static constexpr uint32_t idesc_re_im = idesc_tf32(BM, 2 * BN);
+};
 
 // Tile slots of one stage.  OP_C: 0 A (raw, then hi), 1 A lo, 2 B (raw, then
 // hi), 3 B1 hi, 4 B lo, 5 B1 lo ([B; B1] hi and lo each 256 contiguous
 // rows).  OP_N: 0 A raw (16 x 256 words, row-major, unswizzled), 1 B (raw,
 // then hi), 2 B lo, 3 A0 hi, 4 A0 lo, 5 A1 hi, 6 A1 lo.
-template <int OP>
+// Byte offsets of the slots.
+template <int OP, int BN>
 struct Slots {
   static constexpr bool kC = OP == QEB_OP_C;
-  static constexpr int tiles = kC ? 6 : 7;
-  static constexpr int stage_bytes = tiles * TILE;
-  static constexpr int raw_a = 0, raw_b = kC ? 2 : 1;
-  static constexpr int a_re_hi = kC ? 0 : 3, a_re_lo = kC ? 1 : 4;
-  static constexpr int a_im_hi = kC ? 0 : 5, a_im_lo = kC ? 1 : 6;
-  static constexpr int b_re_hi = kC ? 2 : 1, b_re_lo = kC ? 4 : 2;
-  static constexpr int b_im_hi = kC ? 3 : 1, b_im_lo = kC ? 5 : 2;
-  static_assert(!kC || (b_im_hi == b_re_hi + 1 && b_im_lo == b_re_lo + 1),
-                "[B; B1] contiguous for the N256 product");
+  static constexpr int bt = Shape<BN>::b_tile;
+  static constexpr int stage_bytes = kC ? 2 * TILE + 4 * bt : 5 * TILE + 2 * bt;
+  static constexpr int raw_a = 0, raw_b = kC ? 2 * TILE : TILE;
+  static constexpr int a_first = TILE + 2 * bt;  // OP_N: A0 and A1
+  static constexpr int a_re_hi = kC ? 0 : a_first, a_re_lo = kC ? TILE : a_first + TILE;
+  static constexpr int a_im_hi = kC ? 0 : a_first + 2 * TILE;
+  static constexpr int a_im_lo = kC ? TILE : a_first + 3 * TILE;
+  static constexpr int b_re_hi = raw_b, b_re_lo = raw_b + (kC ? 2 * bt : bt);
+  static constexpr int b_im_hi = kC ? b_re_hi + bt : b_re_hi;
+  static constexpr int b_im_lo = kC ? b_re_lo + bt : b_re_lo;
 };
 
-template <int OP>
+template <int OP, int BN>
 constexpr size_t smem_bytes() {
-  return (size_t)STAGES * Slots<OP>::stage_bytes + 1024 /*alignment*/ + 256 /*barriers*/;
+  return (size_t)STAGES * Slots<OP, BN>::stage_bytes + 1024 /*alignment*/ + 256 /*barriers*/;
 }
 
 struct Maps {
@@ -104,14 +118,15 @@ __device__ __forceinline__ float4 lo4(float4 v, float4 h) {
                      tf32_round(v.w - h.w));
 }
 
-// Split one K-major tile in place (hi) with its lo part into another slot.
+// Split one K-major tile of BYTES in place (hi) with its lo part into another slot.
 // The split is elementwise, so the 128-byte swizzle needs no attention.
+template <int BYTES>
 __device__ __forceinline__ void split_tile(unsigned char* tile, unsigned char* lo, int ct,
                                            unsigned char* swap_hi, unsigned char* swap_lo) {
   float4* t = reinterpret_cast<float4*>(tile);
   float4* l = reinterpret_cast<float4*>(lo);
 #pragma unroll 2
-  for (int c = ct; c < TILE / 16; c += WORKER_THREADS) {
+  for (int c = ct; c < BYTES / 16; c += WORKER_THREADS) {
     const float4 v = t[c];
     const float4 h = hi4(v), w = lo4(v, h);
     t[c] = h;
@@ -146,19 +161,21 @@ __device__ __forceinline__ void transpose_a(const unsigned char* raw, unsigned c
 }
 
 // Worker side of one stage's accumulator buffer: wait until its MMAs are
-// done, add Re (columns [0, 64) of this warp's half) and Im into registers,
+// done, add Re (this warp's half of the columns) and Im into registers,
 // release the buffer.  False on a timed-out wait.
+template <int BN>
 __device__ __forceinline__ bool drain_accumulator(float (&acc)[BN], uint64_t* acc_full,
                                                   uint64_t* acc_empty, int i, uint32_t lane_base,
                                                   int lane) {
   const int b = i & 1;
   if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (i >> 1) & 1))) return false;
   asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t t = lane_base + b * ACC_COLS;
+  const uint32_t t = lane_base + b * Shape<BN>::acc_cols;
+  constexpr int kHalf = BN / 64;  // 32-column loads of Re, then of Im
 #pragma unroll
-  for (int part = 0; part < 4; ++part) {  // Re 0-31, Re 32-63, Im 0-31, Im 32-63
+  for (int part = 0; part < 2 * kHalf; ++part) {
     float v[32];
-    tmem_ld32(t + (part >> 1) * BN + (part & 1) * 32, v);
+    tmem_ld32(t + (part / kHalf) * BN + (part % kHalf) * 32, v);
     tmem_wait_ld();
 #pragma unroll
     for (int j = 0; j < 32; ++j) acc[part * 32 + j] += v[j];
@@ -169,7 +186,7 @@ __device__ __forceinline__ bool drain_accumulator(float (&acc)[BN], uint64_t* ac
   return true;
 }
 
-template <int OP, bool TAIL = false>
+template <int OP, int BN, bool TAIL = false>
 __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
     const __grid_constant__ Maps maps, int M, int N, int kb_per_split, int kb_total, float2 alpha,
     float2 beta, float2* C, int64_t ldc, float2* split, int* error, int skip_m, int skip_n,
@@ -179,7 +196,8 @@ __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
   // TAIL: grid (tail tiles, 1, K slices) over rows m_off + x of column
   // n_off; the K slices go to compact BM x BN partial tiles.
   if (!TAIL && (int)blockIdx.y == skip_n && (int)blockIdx.x >= skip_m) return;
-  using S = Slots<OP>;
+  using S = Slots<OP, BN>;
+  using W = Shape<BN>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -216,7 +234,7 @@ __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS));
+                 "r"(W::tmem_cols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -235,14 +253,14 @@ __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
         }
         if (*abort_v) break;
         unsigned char* st = base + s * S::stage_bytes;
-        mbar_expect_tx(&full[s], 2 * TILE);
+        mbar_expect_tx(&full[s], TILE + S::bt);
         const int kb = kb0 + i;
         if (OP == QEB_OP_C) {
-          tma_load_2d(st + S::raw_a * TILE, &maps.a, &full[s], kb * BKF, m0);
+          tma_load_2d(st + S::raw_a, &maps.a, &full[s], kb * BKF, m0);
         } else {
-          tma_load_2d(st + S::raw_a * TILE, &maps.a, &full[s], 2 * m0, kb * (BKF / 2));
+          tma_load_2d(st + S::raw_a, &maps.a, &full[s], 2 * m0, kb * (BKF / 2));
         }
-        tma_load_2d(st + S::raw_b * TILE, &maps.b, &full[s], kb * BKF, n0);
+        tma_load_2d(st + S::raw_b, &maps.b, &full[s], kb * BKF, n0);
         if (i + kPrefetch < nk) {  // the tiles of stage i + kPrefetch into L2
           const int kp = kb + kPrefetch;
           if (OP == QEB_OP_C)
@@ -266,32 +284,32 @@ __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t st = smem_u32(base + s * S::stage_bytes);
-        const uint32_t t_re = tmem + b * ACC_COLS, t_im = t_re + BN;
+        const uint32_t t_re = tmem + b * W::acc_cols, t_im = t_re + BN;
 #pragma unroll
         for (int kk = 0; kk < BKF / 8; ++kk) {
           const uint32_t off = kk * 32;  // 8 tf32 words along K
           const uint32_t acc = kk > 0 ? 1u : 0u;
-          const uint64_t arh = smem_desc_sw128(st + S::a_re_hi * TILE + off);
-          const uint64_t arl = smem_desc_sw128(st + S::a_re_lo * TILE + off);
-          const uint64_t aih = smem_desc_sw128(st + S::a_im_hi * TILE + off);
-          const uint64_t ail = smem_desc_sw128(st + S::a_im_lo * TILE + off);
-          const uint64_t brh = smem_desc_sw128(st + S::b_re_hi * TILE + off);
-          const uint64_t brl = smem_desc_sw128(st + S::b_re_lo * TILE + off);
-          const uint64_t bih = smem_desc_sw128(st + S::b_im_hi * TILE + off);
-          const uint64_t bil = smem_desc_sw128(st + S::b_im_lo * TILE + off);
+          const uint64_t arh = smem_desc_sw128(st + S::a_re_hi + off);
+          const uint64_t arl = smem_desc_sw128(st + S::a_re_lo + off);
+          const uint64_t aih = smem_desc_sw128(st + S::a_im_hi + off);
+          const uint64_t ail = smem_desc_sw128(st + S::a_im_lo + off);
+          const uint64_t brh = smem_desc_sw128(st + S::b_re_hi + off);
+          const uint64_t brl = smem_desc_sw128(st + S::b_re_lo + off);
+          const uint64_t bih = smem_desc_sw128(st + S::b_im_hi + off);
+          const uint64_t bil = smem_desc_sw128(st + S::b_im_lo + off);
           if constexpr (OP == QEB_OP_C) {
             // [B; B1] from the B slot: Re columns t_re .. +127, Im t_im .. +127
-            mma_tf32(t_re, arh, brh, kIdescReIm, acc);
-            mma_tf32(t_re, arh, brl, kIdescReIm, 1u);
-            mma_tf32(t_re, arl, brh, kIdescReIm, 1u);
+            mma_tf32(t_re, arh, brh, W::idesc_re_im, acc);
+            mma_tf32(t_re, arh, brl, W::idesc_re_im, 1u);
+            mma_tf32(t_re, arl, brh, W::idesc_re_im, 1u);
             (void)aih, (void)ail, (void)bih, (void)bil;
           } else {
-            mma_tf32(t_re, arh, brh, kIdesc, acc);
-            mma_tf32(t_re, arh, brl, kIdesc, 1u);
-            mma_tf32(t_re, arl, brh, kIdesc, 1u);
-            mma_tf32(t_im, aih, bih, kIdesc, acc);
-            mma_tf32(t_im, aih, bil, kIdesc, 1u);
-            mma_tf32(t_im, ail, bih, kIdesc, 1u);
+            mma_tf32(t_re, arh, brh, W::idesc, acc);
+            mma_tf32(t_re, arh, brl, W::idesc, 1u);
+            mma_tf32(t_re, arl, brh, W::idesc, 1u);
+            mma_tf32(t_im, aih, bih, W::idesc, acc);
+            mma_tf32(t_im, aih, bil, W::idesc, 1u);
+            mma_tf32(t_im, ail, bih, W::idesc, 1u);
           }
         }
         mma_commit(&empty[s]);     // the stage may be reloaded
@@ -306,7 +324,7 @@ __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
     const int quarter = warp & 3;             // tensor-memory lane window
     const int half = (warp - 2) >> 2;         // column half of Re and Im
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + half * (BN / 2);
-    float acc[BN];                            // Re [0, 64), Im [64, 128) of this row
+    float acc[BN];                            // Re, then Im, of this row's half
 #pragma unroll
     for (int j = 0; j < BN; ++j) acc[j] = 0.0f;
     bool ok = true;
@@ -318,20 +336,20 @@ __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
       }
       unsigned char* st = base + s * S::stage_bytes;
       if (OP == QEB_OP_C) {
-        split_tile(st + S::raw_a * TILE, st + S::a_re_lo * TILE, ct, nullptr, nullptr);
-        split_tile(st + S::raw_b * TILE, st + S::b_re_lo * TILE, ct, st + S::b_im_hi * TILE,
-                   st + S::b_im_lo * TILE);
+        split_tile<TILE>(st + S::raw_a, st + S::a_re_lo, ct, nullptr, nullptr);
+        split_tile<S::bt>(st + S::raw_b, st + S::b_re_lo, ct, st + S::b_im_hi,
+                   st + S::b_im_lo);
       } else {
-        transpose_a(st + S::raw_a * TILE, st + S::a_re_hi * TILE, st + S::a_re_lo * TILE,
-                    st + S::a_im_hi * TILE, st + S::a_im_lo * TILE, ct);
-        split_tile(st + S::raw_b * TILE, st + S::b_re_lo * TILE, ct, nullptr, nullptr);
+        transpose_a(st + S::raw_a, st + S::a_re_hi, st + S::a_re_lo,
+                    st + S::a_im_hi, st + S::a_im_lo, ct);
+        split_tile<S::bt>(st + S::raw_b, st + S::b_re_lo, ct, nullptr, nullptr);
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&conv[s]);
-      if (i > 0 && !drain_accumulator(acc, acc_full, acc_empty, i - 1, lane_base, lane)) ok = false;
+      if (i > 0 && !drain_accumulator<BN>(acc, acc_full, acc_empty, i - 1, lane_base, lane)) ok = false;
     }
-    if (ok && nk > 0 && !drain_accumulator(acc, acc_full, acc_empty, nk - 1, lane_base, lane))
+    if (ok && nk > 0 && !drain_accumulator<BN>(acc, acc_full, acc_empty, nk - 1, lane_base, lane))
       ok = false;
     if (!ok && lane == 0) {
       atomicExch(error, 13);
@@ -386,7 +404,7 @@ __global__ void __launch_bounds__(THREADS, 1) cgemm_tf32x3_kernel(
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(TMEM_COLS));
+                 "r"(W::tmem_cols));
   }
 }
 
@@ -417,7 +435,7 @@ __global__ void reduce_slices(int M, int N, int splits, const float2* __restrict
 // C = alpha * sum_s P[s] + beta * C over the ntiles tail tiles (rows m_off ..
 // m_off + ntiles - 1 of tile column n_off): compact partial tiles
 // P[(s * ntiles + t) * BM * BN + r + c * BM], slices summed in ascending order.
-__global__ void reduce_tail(int M, int N, int splits, int m_off, int n_off, int ntiles,
+__global__ void reduce_tail(int M, int N, int BN, int splits, int m_off, int n_off, int ntiles,
                             const float2* __restrict__ P, float2 alpha, float2 beta, float2* C,
                             int64_t ldc) {
   const int64_t per_tile = (int64_t)BM * BN;
@@ -482,6 +500,7 @@ int sm_count() {
 // (for 8 tiles, 152 CTAs on 148 SMs), and measured two-wave splits were
 // 25-30 % faster on the Davidson overlaps (K = 80 725).
 int choose_splits(int M, int N, int K) {
+  const int BN = tile_columns(N);
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int kblocks = (2 * K + BKF - 1) / BKF;
   int s = (2 * sm_count()) / tiles;
@@ -497,6 +516,7 @@ int choose_splits(int M, int N, int K) {
 // (reduced afterwards), instead of leaving most SMs idle for a whole wave.
 // Returns the tail's slice count (0: no tail split) and its scratch bytes.
 int tail_splits(int M, int N, int K, int64_t* bytes) {
+  const int BN = tile_columns(N);
   const int mt = (M + BM - 1) / BM;
   const int tiles = mt * ((N + BN - 1) / BN);
   const int sm = sm_count();
@@ -513,11 +533,11 @@ int tail_splits(int M, int N, int K, int64_t* bytes) {
   return ts;
 }
 
-template <int OP>
+template <int OP, int BN>
 int launch(const Maps& maps, int M, int N, int K, float2 al, float2 be, float2* C, int64_t ldc,
            void* scratch, int64_t scratch_bytes, int requested_splits, int* err, cudaStream_t s) {
-  cudaError_t e = qeb::raise_smem_limit(cgemm_tf32x3_kernel<OP>, smem_bytes<OP>());
-  if (e == cudaSuccess) e = qeb::raise_smem_limit(cgemm_tf32x3_kernel<OP, true>, smem_bytes<OP>());
+  cudaError_t e = qeb::raise_smem_limit(cgemm_tf32x3_kernel<OP, BN>, smem_bytes<OP, BN>());
+  if (e == cudaSuccess) e = qeb::raise_smem_limit(cgemm_tf32x3_kernel<OP, BN, true>, smem_bytes<OP, BN>());
   if (e != cudaSuccess) return qeb::cuda_status(e, "cgemm_tf32x3 shared-memory limit");
   const int kblocks = (2 * K + BKF - 1) / BKF;
   int splits = requested_splits > 0 ? (requested_splits < kblocks ? requested_splits : kblocks)
@@ -530,15 +550,15 @@ int launch(const Maps& maps, int M, int N, int K, float2 al, float2 be, float2* 
       const int rem = (mt * nt) % sm_count();
       float2* part = static_cast<float2*>(scratch);
       // every tile but the tail (the last rem rows of the last tile column), unsplit
-      cgemm_tf32x3_kernel<OP><<<dim3(mt, nt, 1), THREADS, smem_bytes<OP>(), s>>>(
+      cgemm_tf32x3_kernel<OP, BN><<<dim3(mt, nt, 1), THREADS, smem_bytes<OP, BN>(), s>>>(
           maps, M, N, kblocks, kblocks, al, be, C, ldc, nullptr, err, mt - rem, nt - 1, 0, 0, 0);
       const int per_t = (kblocks + ts - 1) / ts;
       ts = (kblocks + per_t - 1) / per_t;
-      cgemm_tf32x3_kernel<OP, true><<<dim3(rem, 1, ts), THREADS, smem_bytes<OP>(), s>>>(
+      cgemm_tf32x3_kernel<OP, BN, true><<<dim3(rem, 1, ts), THREADS, smem_bytes<OP, BN>(), s>>>(
           maps, M, N, per_t, kblocks, al, be, C, ldc, part, err, 0, -1, mt - rem, nt - 1, rem);
       int blocks = (int)(((int64_t)rem * BM * BN + 255) / 256);
       if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-      reduce_tail<<<blocks, 256, 0, s>>>(M, N, ts, mt - rem, nt - 1, rem, part, al, be, C, ldc);
+      reduce_tail<<<blocks, 256, 0, s>>>(M, N, BN, ts, mt - rem, nt - 1, rem, part, al, be, C, ldc);
       qeb::count_launches(3);
       return qeb::cuda_status(cudaGetLastError(), "cgemm_tf32x3 launch");
     }
@@ -552,7 +572,7 @@ int launch(const Maps& maps, int M, int N, int K, float2 al, float2 be, float2* 
   splits = (kblocks + per - 1) / per;
   float2* part = splits > 1 ? static_cast<float2*>(scratch) : nullptr;
   const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, splits);
-  cgemm_tf32x3_kernel<OP><<<grid, THREADS, smem_bytes<OP>(), s>>>(maps, M, N, per, kblocks, al,
+  cgemm_tf32x3_kernel<OP, BN><<<grid, THREADS, smem_bytes<OP, BN>(), s>>>(maps, M, N, per, kblocks, al,
                                                                   be, C, ldc, part, err, 0, -1,
                                                                   0, 0, 0);
   qeb::count_launches(1);
@@ -611,6 +631,7 @@ extern "C" int qeb_cgemm_tf32x3_ex(int op_a, int M, int N, int K, const double* 
     qeb::set_error("cgemm_tf32x3: A and B need 16-byte aligned columns (even leading dimension)");
     return QEB_EUNSUPPORTED;
   }
+  const int BN = tile_columns(N);
   if ((int64_t)2 * K > 0x7fffffff || (int64_t)2 * M > 0x7fffffff || (N + BN - 1) / BN > 65535) {
     qeb::set_error("cgemm_tf32x3: matrix too large for one launch");
     return QEB_EUNSUPPORTED;
@@ -632,7 +653,15 @@ extern "C" int qeb_cgemm_tf32x3_ex(int op_a, int M, int N, int K, const double* 
   const float2 be = make_float2((float)beta[0], (float)beta[1]);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float2* c = static_cast<float2*>(C);
-  return op_a == QEB_OP_C
-             ? launch<QEB_OP_C>(maps, M, N, K, al, be, c, ldc, scratch, scratch_bytes, splits, err, s)
-             : launch<QEB_OP_N>(maps, M, N, K, al, be, c, ldc, scratch, scratch_bytes, splits, err, s);
+  auto run = [&](auto op, auto columns) {
+    return launch<decltype(op)::value, decltype(columns)::value>(maps, M, N, K, al, be, c, ldc,
+                                                                 scratch, scratch_bytes, splits,
+                                                                 err, s);
+  };
+  using Adjoint = std::integral_constant<int, QEB_OP_C>;
+  using Plain = std::integral_constant<int, QEB_OP_N>;
+  using Narrow = std::integral_constant<int, 64>;
+  using Wide = std::integral_constant<int, 128>;
+  if (op_a == QEB_OP_C) return BN == 64 ? run(Adjoint{}, Narrow{}) : run(Adjoint{}, Wide{});
+  return BN == 64 ? run(Plain{}, Narrow{}) : run(Plain{}, Wide{});
 }
