@@ -339,8 +339,8 @@ int line_keep(int n, int reach) {
 int line_columns(const qeb_local_plan* p) {
   int x1, x2, y1, y2;
   if (!line_split(p->nx, &x1, &x2) || !line_split(p->ny, &y1, &y2)) return 0;
-  return p->precision == QEB_F64 ? lines::plane_columns<double>(x1, x2, y1, y2, p->line_rows)
-                                 : lines::plane_columns<float>(x1, x2, y1, y2, p->line_rows);
+  return p->precision == QEB_F64 ? lines::plane_columns<double>(x1, x2, y1, y2, p->line_rows, false)
+                                 : lines::plane_columns<float>(x1, x2, y1, y2, p->line_rows, false);
 }
 
 int lines_prepare(const qeb_local_plan* p) {

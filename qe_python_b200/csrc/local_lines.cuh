@@ -287,7 +287,21 @@ constexpr size_t plane_smem(int x1, int x2, int y1, int y2, int rows, int column
 }
 
 constexpr size_t kMaxSmem = 227 * 1024, kSmemPerSm = 228 * 1024;
-constexpr int kPlaneThreads = 512;  // most threads of a plane block
+
+// Launch bounds of a plane kernel: most threads per block and blocks per SM that
+// its registers allow (FP32 64 per thread; FP64 80 up to DFT10, where three
+// blocks of 256 threads measured faster than two, 64^3 0.387 -> 0.358 ms and
+// 90^3 0.535 -> 0.491, and 128 for longer DFTs, which spill below that: 135^3
+// 1.83 ms at 128, 2.68 at 80).  The run-time kernel holds every length.
+struct PlaneBounds {
+  int threads, blocks;
+};
+template <typename T>
+constexpr PlaneBounds plane_bounds(int x1, int x2, int y1, int y2, bool compiled) {
+  if (sizeof(T) == 4) return {512, 2};
+  const bool small = x1 <= 10 && x2 <= 10 && y1 <= 10 && y2 <= 10;
+  return compiled && small ? PlaneBounds{384, 2} : PlaneBounds{512, 1};
+}
 
 // Relative time of a plane with `columns` columns per batch and t threads,
 // `resident` blocks per SM at most: every step's rounds of t small DFTs, each
@@ -299,12 +313,12 @@ constexpr int kPlaneThreads = 512;  // most threads of a plane block
 // second within 4 % rms, where the timings of one length span up to 1.4 x).
 template <typename T>
 constexpr double plane_cost(int x1, int x2, int y1, int y2, int rows, int columns, int t,
-                            int resident, double whole) {
+                            int budget, int resident, double whole) {
   constexpr bool single = sizeof(T) == 4;
   const int ny = y1 * y2, batches = (ny + columns - 1) / columns;
   const int by_smem =
       (int)(kSmemPerSm / (plane_smem<T>(x1, x2, y1, y2, rows, columns) + 1024));
-  int blocks = (single ? 1024 : 512) / t;  // by registers
+  int blocks = budget / t;  // by registers
   blocks = blocks < by_smem ? blocks : by_smem;
   blocks = blocks < resident ? blocks : resident;
   if (blocks < 1) blocks = 1;
@@ -321,17 +335,19 @@ constexpr double kWholeRounds = sizeof(T) == 4 ? 0.0 : 0.4;
 
 // Columns of one batch, by the cost above; 0: the plane does not fit.
 template <typename T>
-constexpr int plane_columns(int x1, int x2, int y1, int y2, int rows) {
+constexpr int plane_columns(int x1, int x2, int y1, int y2, int rows, bool compiled) {
   const int ny = y1 * y2;
+  const PlaneBounds bounds = plane_bounds<T>(x1, x2, y1, y2, compiled);
+  const int budget = bounds.threads * bounds.blocks;
   int best = 0;
   double best_cost = 0.0;
   for (int batches = 1; batches <= ny; ++batches) {
     const int columns = (ny + batches - 1) / batches;
     if (batches > 8 && best > 0) break;
     if (plane_smem<T>(x1, x2, y1, y2, rows, columns) > kMaxSmem) continue;
-    for (int t = 64; t <= kPlaneThreads; t += 32) {
+    for (int t = 64; t <= bounds.threads; t += 32) {
       const double cost =
-          plane_cost<T>(x1, x2, y1, y2, rows, columns, t, 32, kWholeRounds<T>);
+          plane_cost<T>(x1, x2, y1, y2, rows, columns, t, budget, 32, kWholeRounds<T>);
       if (best == 0 || cost < best_cost) best = columns, best_cost = cost;
     }
   }
@@ -345,11 +361,13 @@ int plane_threads(const P& g, int64_t blocks) {
   const int64_t per_sm = (blocks + 147) / 148;
   const int resident = per_sm < 32 ? (int)per_sm : 32;
   const double whole = per_sm < 2 ? 1.0 : kWholeRounds<T>;
+  const PlaneBounds bounds = plane_bounds<T>(g.x1, g.x2, g.y1, g.y2, P::kStatic);
+  const int budget = bounds.threads * bounds.blocks;
   int best = 64;
   double best_cost = 0.0;
-  for (int t = 64; t <= kPlaneThreads; t += 32) {
+  for (int t = 64; t <= bounds.threads; t += 32) {
     const double cost =
-        plane_cost<T>(g.x1, g.x2, g.y1, g.y2, g.rows, g.columns, t, resident, whole);
+        plane_cost<T>(g.x1, g.x2, g.y1, g.y2, g.rows, g.columns, t, budget, resident, whole);
     if (t == 64 || cost < best_cost) best = t, best_cost = cost;
   }
   return best;
@@ -365,7 +383,7 @@ RuntimePlane runtime_plane(const qeb_local_plan* p, int rows) {
   g.stride = p->ny | 1;
   g.rows = rows;
   g.columns = rows == p->line_rows ? p->line_columns
-                                   : plane_columns<T>(g.x1, g.x2, g.y1, g.y2, rows);
+                                   : plane_columns<T>(g.x1, g.x2, g.y1, g.y2, rows, false);
   return g;
 }
 

@@ -12,12 +12,16 @@
 namespace qeb {
 namespace lines {
 
-// Registers of a plane thread: 64 (FP32: two blocks of 512 threads), 128 (FP64).
-template <typename T>
-constexpr int kMinBlocks = sizeof(T) == 4 ? 2 : 1;
+template <typename T, class P>
+constexpr PlaneBounds bounds_of() {
+  if constexpr (P::kStatic)
+    return plane_bounds<T>(P::x1, P::x2, P::y1, P::y2, true);
+  else
+    return plane_bounds<T>(16, 16, 16, 16, false);
+}
 
 template <typename T, int MODE, class P>
-__global__ void __launch_bounds__(kPlaneThreads, kMinBlocks<T>) plane_kernel(
+__global__ void __launch_bounds__((bounds_of<T, P>().threads), (bounds_of<T, P>().blocks)) plane_kernel(
     const __grid_constant__ KBatch<T> kb, const __grid_constant__ P g, int nz, const C2<T>* tw_x,
     const C2<T>* tw_y, const T* potential, const __grid_constant__ DensityTarget rho) {
   const KDesc<T>& d = kb.k[blockIdx.z];
@@ -44,7 +48,7 @@ template <typename T, int MODE, int N1, int N2, int K>
 int launch_static(const KBatch<T>& kb, const qeb_local_plan* p, int nk, int nb, const C2<T>* tw_x,
                   const C2<T>* tw_y, const T* potential, const DensityTarget& rho,
                   cudaStream_t s) {
-  using P = StaticPlane<N1, N2, K, plane_columns<T>(N1, N2, N1, N2, 2 * K * N2)>;
+  using P = StaticPlane<N1, N2, K, plane_columns<T>(N1, N2, N1, N2, 2 * K * N2, true)>;
   return launch_one<T, MODE, P>(kb, P{}, p->nz, nk, nb, tw_x, tw_y, potential, rho, s);
 }
 
@@ -54,11 +58,11 @@ int launch_plane(const KBatch<T>& kb, const qeb_local_plan* p, int nk, int nb,
   const C2<T>* tw_x = tw_at<T>(p, 0);
   const C2<T>* tw_y = tw_at<T>(p, 1);
 #define QEB_CASE(n, a, b, k1, k2)                                                             \
-  if constexpr (plane_columns<T>(a, b, a, b, 2 * k1 * b) > 0) {                               \
+  if constexpr (plane_columns<T>(a, b, a, b, 2 * k1 * b, true) > 0) {                               \
     if (p->nx == n && p->line_k == k1)                                                        \
       return launch_static<T, MODE, a, b, k1>(kb, p, nk, nb, tw_x, tw_y, potential, rho, s);  \
   }                                                                                           \
-  if constexpr (k2 > k1 && plane_columns<T>(a, b, a, b, 2 * k2 * b) > 0) {                    \
+  if constexpr (k2 > k1 && plane_columns<T>(a, b, a, b, 2 * k2 * b, true) > 0) {                    \
     if (p->nx == n && p->line_k == k2)                                                        \
       return launch_static<T, MODE, a, b, k2>(kb, p, nk, nb, tw_x, tw_y, potential, rho, s);  \
   }
