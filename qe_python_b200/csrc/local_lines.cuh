@@ -57,6 +57,7 @@ namespace lines {
 
 constexpr int kSticks = 32;  // sticks of one z block: one lane each
 constexpr int kZThreads = 256;
+constexpr int kAhead = 4;    // entries per thread that a z pass fetches ahead of a barrier
 
 template <typename T>
 struct KDesc {
@@ -168,12 +169,25 @@ __device__ __forceinline__ void z_inverse_body(const KDesc<T>& d, const Z& g,
   const int tid = threadIdx.x, threads = blockDim.x;
   const int s0 = block_x * kSticks;
   const int nsl = min(kSticks, d.nst - s0);
+  // the first entries are on their way while the lines are zeroed
+  const int e0 = d.stick_off[s0], e1 = d.stick_off[s0 + nsl];
+  const C2<T>* col = d.psi + band * d.ld;
+  int pos[kAhead];
+  C2<T> value[kAhead];
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    const int e = e0 + tid + u * threads;
+    pos[u] = e < e1 ? d.entry_pos[e] : -1;
+    if (pos[u] >= 0) value[u] = col[d.entry_g[e]];
+  }
   for (int i = tid; i < g.nz; i += threads) tw[i] = tw_z[(i / g.z1) * (i % g.z1)];
   for (int i = tid; i < kSticks * g.stride; i += threads) lines[i] = mk<T>(0, 0);
-  const int e0 = d.stick_off[s0], e1 = d.stick_off[s0 + nsl];
   __syncthreads();
-  const C2<T>* col = d.psi + band * d.ld;
-  for (int e = e0 + tid; e < e1; e += threads) lines[d.entry_pos[e]] = col[d.entry_g[e]];
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (pos[u] >= 0) lines[pos[u]] = value[u];
+  for (int e = e0 + tid + kAhead * threads; e < e1; e += threads)
+    lines[d.entry_pos[e]] = col[d.entry_g[e]];
   __syncthreads();
   const uint32_t zmask = d.zmask;
   QEB_RADIX(g, z1, [&](auto r) {
@@ -253,11 +267,33 @@ __device__ __forceinline__ void z_forward_body(const KDesc<T>& d, const Z& g,
         if ((zmask >> i) & 1u) p[i * g.z2] = v[i];
     }
   });
-  __syncthreads();
   const int e0 = d.stick_off[s0], e1 = d.stick_off[s0 + nsl];
   const C2<T>* col = d.psi + band * d.ld;
   C2<T>* dst = d.out + band * d.ldo;
-  for (int e = e0 + tid; e < e1; e += threads) {
+  // the first entries' operands are on their way during the barrier
+  int index[kAhead], pos[kAhead];
+  C2<T> own[kAhead];
+  T kinetic[kAhead];
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    const int e = e0 + tid + u * threads;
+    index[u] = e < e1 ? d.entry_g[e] : -1;
+    if (index[u] < 0) continue;
+    pos[u] = d.entry_pos[e];
+    if (d.kinetic != nullptr) {
+      kinetic[u] = d.kinetic[index[u]];
+      own[u] = col[index[u]];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    if (index[u] < 0) continue;
+    C2<T> v = scale(lines[pos[u]], inv_n);
+    if (d.kinetic != nullptr) v = add_scaled(v, kinetic[u], own[u]);
+    dst[index[u]] = v;
+  }
+  for (int e = e0 + tid + kAhead * threads; e < e1; e += threads) {
     const int gi = d.entry_g[e];
     C2<T> v = scale(lines[d.entry_pos[e]], inv_n);
     if (d.kinetic != nullptr) v = add_scaled(v, d.kinetic[gi], col[gi]);
@@ -445,18 +481,15 @@ __device__ __forceinline__ void plane_body(const KDesc<T>& d, const P& g, int nz
   C2<T>* twy_fwd = twy_inv + g.y2 * even(g.y1);
   C2<T>* buf = twy_inv + twiddle_values(g.y1, g.y2);
   C2<T>* plane = buf + g.nx * g.columns;
-  load_twiddles(twx_inv, twx_fwd, tw_x, g.x1, g.x2);
-  load_twiddles(twy_inv, twy_fwd, tw_y, g.y1, g.y2);
-  __syncthreads();
   C2<T>* srow = d.sticks + (band * nz + z) * (int64_t)d.nst;
   const unsigned rinv = inverse_of(rows), cinv = inverse_of(g.columns);
-  // rows 1
+  // rows 1; the first DFT's sticks are on their way while the tables load
   QEB_RADIX(g, y1, [&](auto r) {
     constexpr int R = decltype(r)::value;
-    for (int t = tid; t < g.y2 * rows; t += threads) {
-      const int j = quotient(t, rinv), a = t - j * rows;
+    const int total = g.y2 * rows;
+    C2<T> v[R];
+    auto fetch = [&](int t) {
       int idx[R];
-      C2<T> v[R];
 #pragma unroll
       for (int i = 0; i < R; ++i)
         idx[i] = P::keep_y(d, i) ? __ldg(d.stick_map + t + i * g.y2 * rows) : -1;
@@ -465,6 +498,14 @@ __device__ __forceinline__ void plane_body(const KDesc<T>& d, const P& g, int nz
         v[i] = mk<T>(0, 0);
         if (P::keep_y(d, i) && idx[i] >= 0) v[i] = srow[idx[i]];
       }
+    };
+    if (tid < total) fetch(tid);
+    load_twiddles(twx_inv, twx_fwd, tw_x, g.x1, g.x2);
+    load_twiddles(twy_inv, twy_fwd, tw_y, g.y1, g.y2);
+    __syncthreads();
+    for (int t = tid; t < total; t += threads) {
+      if (t != tid) fetch(t);
+      const int j = quotient(t, rinv), a = t - j * rows;
       dft<T, R, true, Z>(v);
       C2<T>* o = plane + a * g.stride + j * R;
       C2<T> w[even(R)];
