@@ -91,10 +91,9 @@ def parse_args():
     return p.parse_args()
 
 
-# DRAM bytes (read + write) of one pass-B launch of the 256-band microbenchmark,
-# from one ncu capture (--set full) of `bench.py --apply-only f32` (the pruned
-# plane pass, two bands per block): 78.8 MB read + 22.0 MB written.
-PASS_B_NCU_TRAFFIC = {("pass_b", 256): 100.83e6}
+# DRAM bytes (read + write) of one plane-pass launch of the 256-band
+# microbenchmark operator, from one ncu capture: 487.2 GB/s over 207.97 us.
+PASS_B_NCU_TRAFFIC = {("pass_b", 256): 101.33e6}
 
 
 # How the SCF benchmark cells differ from the configurations they stand for:
@@ -710,8 +709,8 @@ def run_b200(args) -> None:
                     "traffic": PASS_B_NCU_TRAFFIC.get((dominant, nb)),
                     "algorithmic_bytes": amount,
                     "peak_source": peaks["source"],
-                    "note": "pass B is bound by the shared-memory data path (ncu: L1/TEX "
-                            "91 %, issue 70 % active), not by HBM"}
+                    "note": "pass B is bound by the shared-memory data path (ncu: LSU "
+                            "wavefronts 82 %, issue 71 % active), not by HBM"}
         if dominant == "pass_b":
             roofline["fp32_fft_rate"] = plane_fft_rate(work.shape, nb, seconds)
     elif dominant in ("calbec_gemm", "add_gemm") and forms["mixed"][1].tensor_gemm:

@@ -22,14 +22,14 @@
 //   * twiddle reads are broadcasts from tables laid out [role][k].
 // The steps of one transform are separated by block barriers; several blocks
 // per SM fill them.  The passes are bound by instruction issue and the
-// shared-memory data path together (64 x 64 plane, FP32: 70 % and 76 %), FP64
+// shared-memory data path together (64 x 64 plane, FP32: 71 % and 82 %), FP64
 // planes of 135 points by one resident block's latency.  Measured against
 // lines spread over the lanes of a warp, plane pass: 135^3 of 96 bands FP32
-// 1.313 -> 0.925 ms, FP64 2.627 -> 1.903; 90^3 of 200 bands FP32 0.697 ->
-// 0.547; 64^3 of 256 bands FP32 0.209 -> 0.202, FP64 0.383 -> 0.404; z passes
-// of 64^3 0.055 + 0.053 -> 0.038 + 0.042, of 135^3 FP32 0.143 + 0.171 -> 0.103
+// 1.313 -> 0.887 ms, FP64 2.627 -> 1.866; 90^3 of 200 bands FP32 0.697 ->
+// 0.520; 64^3 of 256 bands FP32 0.209 -> 0.197, FP64 0.383 -> 0.352; z passes
+// of 64^3 0.055 + 0.053 -> 0.034 + 0.041, of 135^3 FP32 0.143 + 0.171 -> 0.105
 // + 0.125; and against the generic Stockham kernels 80^3 of 60 bands FP32 0.992
-// -> 0.119 ms, 45 x 50 x 90 of 37 bands FP64 0.559 -> 0.081.
+// -> 0.114 ms, 45 x 50 x 90 of 37 bands FP64 0.559 -> 0.074.
 //
 // Plane pass, per block one z plane of one band; rows are the occupied x, the
 // contiguous axis is y (sticks are ordered by (y, x), so the lanes of a warp

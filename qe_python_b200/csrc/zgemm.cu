@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, int 
 // of 12 (4 mod 8: the 2 rows x 4 k of a load phase cover all banks), the
 // M-contiguous A of op N is rows of BM values at a stride of BM + 2 (2 mod 8).
 // Measured against the SIMT kernel: the 23 847 x 184 x 184 rotation 0.373 ->
-// 0.219 ms (29.5 TFLOP/s).
+// 0.218 ms (29.6 TFLOP/s).
 constexpr int kMmaK = 8, kMmaStages = 4, kMmaThreads = 128, kMmaStride = kMmaK + 4;
 
 template <int BMT, int BNT, bool CONJ_A>
@@ -532,7 +532,7 @@ __global__ void skinny_reduce(int Mb, int Ns, int splits, const C2<T>* __restric
 // meet in shared memory four columns at a time.  (One thread per row over the
 // whole of K left 2.1 blocks of 256 rows per SM on the 216-atom cell's
 // projector add, 80 725 x 864 x 5 complex64.)  With the kernel above: H|psi> of 5
-// bands of that cell 0.574 -> 0.347 ms.
+// bands of that cell 0.607 -> 0.345 ms.
 template <typename T, int NS, int V>
 __global__ void __launch_bounds__(kSkinnyThreads) skinny_n_kernel(
     int M, int N, int K, C2<T> alpha, const C2<T>* __restrict__ A, int64_t lda,
