@@ -132,6 +132,14 @@ int64_t qeb_density_scratch_bytes(const qeb_local_plan* plan, int64_t nbands);
 int qeb_accumulate_density(const qeb_local_plan* plan, void* scratch, int64_t scratch_bytes,
                            const void* psi, int64_t ld_psi, int64_t nbands,
                            const double* weights, double* density, void* stream);
+/* The same with the grid (qeb_density_grid_bytes bytes, 0: none is used) in a
+ * buffer of its own, so that the scratch is an H|psi>'s; a null or smaller
+ * grid is not used. */
+int64_t qeb_density_grid_bytes(const qeb_local_plan* plan, int64_t nbands);
+int qeb_accumulate_density_grid(const qeb_local_plan* plan, void* scratch, int64_t scratch_bytes,
+                                void* grid, int64_t grid_bytes, const void* psi, int64_t ld_psi,
+                                int64_t nbands, const double* weights, double* density,
+                                void* stream);
 
 /* ------------------------------------------------------------------------
  * Complex GEMM: C = alpha * op(A) * B + beta * C, column-major.

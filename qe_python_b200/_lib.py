@@ -40,9 +40,11 @@ SIGNATURES: list[tuple[str, object, list]] = [
     ("qeb_local_plan_info", _I, [_P, _P, _I]),
     ("qeb_local_scratch_bytes", _L, [_P, _L]),
     ("qeb_density_scratch_bytes", _L, [_P, _L]),
+    ("qeb_density_grid_bytes", _L, [_P, _L]),
     ("qeb_apply_local", _I, [_P, _P, _L, _P, _L, _L, _P, _P, _P, _L, _P]),
     ("qeb_apply_local_profiled", _I, [_P, _P, _L, _P, _L, _L, _P, _P, _P, _L, _P, _P]),
     ("qeb_accumulate_density", _I, [_P, _P, _L, _P, _L, _L, _P, _P, _P]),
+    ("qeb_accumulate_density_grid", _I, [_P, _P, _L, _P, _L, _P, _L, _L, _P, _P, _P]),
     ("qeb_local_multi_scratch_bytes", _L, [_I, _P, _P]),
     ("qeb_apply_local_multi", _I, [_I, _P, _P, _L, _P, _P, _P, _P, _P, _P, _P, _P]),
     ("qeb_set_persistent_passes", _I, [_I]),

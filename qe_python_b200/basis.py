@@ -323,7 +323,10 @@ def grid_slots(miller: np.ndarray, shape) -> tuple[np.ndarray, np.ndarray, np.nd
 
 
 class FFTScratchPool:
-    """Grow-only named device scratch shared by workspaces (basis.py:407-454)."""
+    """Grow-only named device scratch shared by workspaces (basis.py:407-454).
+
+    A buffer that is outgrown goes back to the allocator: what records a
+    buffer's address (a captured graph) holds its tensor."""
 
     def __init__(self) -> None:
         self._buffers: dict[tuple[str, torch.device], torch.Tensor] = {}
@@ -556,10 +559,15 @@ class LocalPotentialWorkspace:
         batch = min(max(batch, 1), 65535)
         for start in range(0, nb, batch):
             count = min(batch, nb - start)
-            nbytes = int(lib.qeb_density_scratch_bytes(self._plan, count))
-            scratch = self.scratch_pool.buffer("sticks", nbytes, self.device)
-            status = lib.qeb_accumulate_density(
+            # the grid apart from the sticks: the same bands' H|psi> may be
+            # captured in a graph that holds the stick buffer's address
+            scratch, nbytes = self._scratch(count)
+            grid_bytes = int(lib.qeb_density_grid_bytes(self._plan, count))
+            grid = self.scratch_pool.buffer("density", grid_bytes, self.device) \
+                if grid_bytes else None
+            status = lib.qeb_accumulate_density_grid(
                 self._plan, scratch.data_ptr(), nbytes,
+                0 if grid is None else grid.data_ptr(), grid_bytes,
                 vectors.data_ptr() + start * ld * elem, ld, count,
                 weights.data_ptr() + start * 8, rho.data_ptr(), stream,
             )

@@ -553,6 +553,11 @@ static int64_t density_grid_bytes(const qeb_local_plan* p, int64_t nbands) {
   return p->lines && nbands * points >= kDensityGridPoints ? points * 8 : 0;
 }
 
+extern "C" int64_t qeb_density_grid_bytes(const qeb_local_plan* p, int64_t nbands) {
+  if (p == nullptr || nbands < 0) return -1;
+  return density_grid_bytes(p, nbands);
+}
+
 extern "C" int64_t qeb_density_scratch_bytes(const qeb_local_plan* p, int64_t nbands) {
   if (p == nullptr || nbands < 0) return -1;
   return qeb_local_scratch_bytes(p, nbands) + density_grid_bytes(p, nbands);
@@ -685,29 +690,44 @@ extern "C" int qeb_apply_local_multi(int nk, const qeb_local_plan* const* plans,
   return QEB_OK;
 }
 
-extern "C" int qeb_accumulate_density(const qeb_local_plan* p, void* scratch,
-                                      int64_t scratch_bytes, const void* psi, int64_t ld,
-                                      int64_t nbands, const double* weights, double* density,
-                                      void* stream) {
+extern "C" int qeb_accumulate_density_grid(const qeb_local_plan* p, void* scratch,
+                                           int64_t scratch_bytes, void* grid, int64_t grid_bytes,
+                                           const void* psi, int64_t ld, int64_t nbands,
+                                           const double* weights, double* density, void* stream) {
   int rc = check_call(p, scratch, scratch_bytes, psi, ld, nbands, "accumulate_density");
   if (rc) return rc;
   if (nbands > 0 && (weights == nullptr || density == nullptr)) {
     qeb::set_error("accumulate_density: null weights or density");
     return QEB_EINVAL;
   }
+  const int64_t need = density_grid_bytes(p, nbands);
+  double* rho = static_cast<double*>(grid);
+  if (need == 0 || grid_bytes < need) rho = nullptr;
+  if (reinterpret_cast<uintptr_t>(rho) % sizeof(double) != 0) {
+    qeb::set_error("accumulate_density: the grid must be 8-byte aligned");
+    return QEB_EINVAL;
+  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  double* grid = nullptr;
-  if (density_grid_bytes(p, nbands) > 0 && scratch_bytes >= qeb_density_scratch_bytes(p, nbands))
-    grid = reinterpret_cast<double*>(static_cast<unsigned char*>(scratch) +
-                                     qeb_local_scratch_bytes(p, nbands));
   if (p->precision == QEB_F64) {
-    return launch_density<double>(p, static_cast<C2<double>*>(scratch), grid,
+    return launch_density<double>(p, static_cast<C2<double>*>(scratch), rho,
                                   static_cast<const C2<double>*>(psi), ld, nbands, weights,
                                   density, s);
   }
-  return launch_density<float>(p, static_cast<C2<float>*>(scratch), grid,
+  return launch_density<float>(p, static_cast<C2<float>*>(scratch), rho,
                                static_cast<const C2<float>*>(psi), ld, nbands, weights, density,
                                s);
+}
+
+extern "C" int qeb_accumulate_density(const qeb_local_plan* p, void* scratch,
+                                      int64_t scratch_bytes, const void* psi, int64_t ld,
+                                      int64_t nbands, const double* weights, double* density,
+                                      void* stream) {
+  // the grid behind the sticks, when the scratch holds one
+  const int64_t sticks = qeb_local_scratch_bytes(p, nbands);
+  const bool room = scratch != nullptr && sticks >= 0 && scratch_bytes > sticks;
+  return qeb_accumulate_density_grid(
+      p, scratch, scratch_bytes, room ? static_cast<unsigned char*>(scratch) + sticks : nullptr,
+      room ? scratch_bytes - sticks : 0, psi, ld, nbands, weights, density, stream);
 }
 
 // Same operator as qeb_apply_local, with CUDA events recorded on `stream`

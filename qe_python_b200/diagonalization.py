@@ -402,7 +402,8 @@ class HpsiGraph:
         """``private``: the graph gets its own stick scratch, side stream and
         split-K scratch, so that it can replay concurrently with the other
         private graphs of the same Hamiltonian (by default the graphs of one
-        Hamiltonian share them and must replay one after another)."""
+        Hamiltonian share them and must replay one after another, and not
+        beside other calls on its workspace)."""
         npw = len(ham.basis)
         self.ham = ham
         self.nbands = int(nbands)
@@ -434,6 +435,9 @@ class HpsiGraph:
             with torch.cuda.graph(self.graph, stream=stream if private else None):
                 ham.apply_into(self.input, self.output)
             torch.cuda.synchronize()
+            # the graph recorded this buffer's address; a later call of more
+            # bands replaces it in a shared pool
+            self._sticks = workspace.scratch_pool.buffer("sticks", 0, ham.device)
         finally:
             # the private scratch and side stream stay alive with the graph
             self._scratch_pool, self._side = workspace.scratch_pool, ham._side_stream()
