@@ -52,8 +52,10 @@ __device__ __forceinline__ double block_sum(double v, double* shared) {
   return total;
 }
 
+// Not the .aligned form, which wants every warp converged: thread 0 comes here
+// from branches that it alone takes.
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // The double at `p` of this block's shared memory as block `rank` holds it.
 __device__ __forceinline__ double cluster_read(const double* p, unsigned rank) {
