@@ -260,7 +260,8 @@ int apply_t(int nk, const qeb_local_plan* const* plans, void* const* sticks,
 }
 
 // density[x, y, z] += grid[z, x, y]: 32 x 32 tiles of (y, z) through shared
-// memory, both sides coalesced.
+// memory, both sides coalesced.  Atomic, as the straight form is: calls on
+// several streams, each with scratch of its own, may add to one density.
 __global__ void __launch_bounds__(256) density_add_kernel(int nx, int ny, int nz,
                                                           const double* __restrict__ grid,
                                                           double* __restrict__ density) {
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(256) density_add_kernel(int nx, int ny, int nz
   __syncthreads();
   for (int j = ty; j < 32; j += 8)
     if (y0 + j < ny && z0 + tx < nz)
-      density[((int64_t)x * ny + y0 + j) * nz + z0 + tx] += tile[tx][j];
+      atomicAdd(density + ((int64_t)x * ny + y0 + j) * nz + z0 + tx, tile[tx][j]);
 }
 
 // grid: nx ny nz doubles of scratch in which the bands' contributions are
