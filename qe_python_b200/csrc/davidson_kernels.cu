@@ -157,30 +157,8 @@ __device__ __forceinline__ void for_runs(int64_t rows, int64_t first, Fn&& fn) {
   }
 }
 
-// 2 / d with d = (1 + x + sqrt(1 + (x - 1)^2)) / 2.  For complex64 vectors the
-// square root and the quotient come from the hardware's approximations refined
-// by Newton steps (relative error below 1e-13, far under the rounding of the
-// result to 24 bits): the full FP64 routines on every element were half
-// of the kernel's time.
-template <typename T>
-__device__ __forceinline__ double precondition_factor(double x) {
-  const double a = fma(x - 1.0, x - 1.0, 1.0);
-  if (sizeof(T) == 4 && a < 1.0e300) {
-    double y, r;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    double root = a * y;
-    root = fma(0.5 * y, fma(-root, root, a), root);
-    root = fma(0.5 * y, fma(-root, root, a), root);  // 1 + x + root cancels for x << 0
-    const double d = 0.5 * (1.0 + x + root);
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    r = fma(r, fma(-d, r, 1.0), r);
-    return 2.0 * r;
-  }
-  const double d = 0.5 * (1.0 + x + sqrt(a));
-  return 2.0 / d;
-}
-
-// x = 2 (H_GG - e_b) [Ry], out = 2 r / d
+// x = 2 (H_GG - e_b) [Ry], d = (1 + x + sqrt(1 + (x - 1)^2)) / 2, out = 2 r / d,
+// in FP64 whatever the vectors' precision.
 template <typename T, int V>
 __global__ void __launch_bounds__(kRunThreads) precondition_kernel(
     int64_t rows, int64_t blocks, const C2<T>* __restrict__ r, int64_t ldr,
@@ -196,7 +174,9 @@ __global__ void __launch_bounds__(kRunThreads) precondition_kernel(
     load_run<T, W>(v, src + g);
 #pragma unroll
     for (int i = 0; i < W; ++i) {
-      const double s = precondition_factor<T>(2.0 * (diag[g + i] - eb));
+      const double x = 2.0 * (diag[g + i] - eb);
+      const double d = 0.5 * (1.0 + x + sqrt(1.0 + (x - 1.0) * (x - 1.0)));
+      const double s = 2.0 / d;
       v[i] = qeb::mk<T>((T)(s * (double)v[i].re), (T)(s * (double)v[i].im));
     }
     store_run<T, W>(dst + g, v);
