@@ -99,16 +99,19 @@ __global__ void __launch_bounds__(kReduceThreads) column_reduce(
   };
   constexpr int kStep = kReduceThreads * V;
   int64_t g = first + threadIdx.x * V;
-  // four runs in flight per thread (their sums stay in row order)
-  for (; g + 3 * kStep + V <= last; g += 4 * kStep) {
-    C2<T> a[4][V], b[4][V];
+  // four loads in flight per thread, two from each operand of an inner product
+  // (four from each took 160 us on 50 000 x 480 complex128, two 118), the
+  // sums in row order
+  constexpr int kRuns = MODE == 2 ? 2 : 4;
+  for (; g + (kRuns - 1) * kStep + V <= last; g += kRuns * kStep) {
+    C2<T> a[kRuns][V], b[kRuns][V];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < kRuns; ++u) {
       load_run<T, V>(a[u], l + g + u * kStep);
       if constexpr (MODE == 2) load_run<T, V>(b[u], r + g + u * kStep);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < kRuns; ++u)
 #pragma unroll
       for (int v = 0; v < V; ++v) add(g + u * kStep + v, a[u][v], MODE == 2 ? b[u][v] : a[u][v]);
   }
@@ -247,9 +250,16 @@ int64_t run_blocks(int64_t rows, int64_t cols, int64_t* per_column) {
 template <typename T, int MODE>
 int launch_reduce(int64_t rows, int64_t cols, const void* left, int64_t ldl, const void* right,
                   int64_t ldr, const double* diag, double* out, cudaStream_t stream) {
-  // blocks per column: about four per SM in all, each with at least 4096 rows
+  // blocks per column: about four per SM in all for complex64 values, three for
+  // complex128, each with at least 4096 rows, or 8192 once there are three per SM.
+  // Columns that fill the GPU alone stay whole (squared norms, one block a column
+  // against two: 80 725 x 480 complex128 97 and 109 us, 11 019 x 480 complex64 8.6
+  // and 10.6); fewer gain by the split (80 725 x 131 complex128, one and four, 57 and 31).
+  constexpr int kFill = (sizeof(T) == 4 ? 4 : 3) * 148;
   int parts = 1;
-  while (parts < kMaxCluster && cols * parts < 4 * 148 && rows / (2 * parts) >= 4096) parts *= 2;
+  while (parts < kMaxCluster && cols * parts < kFill &&
+         rows / (2 * parts) >= (cols * parts < 3 * 148 ? 4096 : 8192))
+    parts *= 2;
   int64_t part_rows = (rows + parts - 1) / parts;
   part_rows = (part_rows + 1) & ~int64_t(1);  // every part starts on a whole run
   if (cols * parts > 0x7fffffff) {

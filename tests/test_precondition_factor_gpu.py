@@ -11,9 +11,10 @@ pytestmark = pytest.mark.gpu
 def test_factor_is_rounded_in_fp64(cuda_device):
     """The products' roundings to 24 bits against a NumPy FP64 factor.  Two
     factors r apart (relative) round a product to different values for a share
-    of about r / 2^-24 of the components: a factor good to 1e-12 shows in some 70
-    of the 4 million here, the last bits in which two FP64 evaluations differ
-    (3e-16 on these x, about 2e-8 per component) in none or one."""
+    of about r / 2^-24 of the components: a factor good to 1e-13 shows in some 7
+    of the 4 million here (six were seen of approximate reciprocals with Newton
+    steps), the last bits in which two FP64 evaluations differ (3e-16 on these
+    x, about 5e-9 per component) in none."""
     import torch
 
     from qe_python_b200 import kernels as K
