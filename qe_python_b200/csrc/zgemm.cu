@@ -336,7 +336,7 @@ __global__ void reduce_partials(int M, int N, int splits, const C2<T>* __restric
 // Skinny products: one side of the output has at most 16 columns.  The tiled
 // kernel above wastes most of a 64-wide tile there and reads the large
 // operand once per tile column; these kernels stream the large operand once
-// from HBM and keep the narrow one in shared memory.  Cases of the hot path:
+// from HBM.  Cases of the hot path:
 // calbec and the projector add for a few unconverged bands, the Davidson
 // rows of a few correction vectors (new^H [HV, V]) and their Ritz columns.
 
@@ -600,6 +600,134 @@ __global__ void __launch_bounds__(kSkinnyThreads) skinny_n_kernel(
 }
 static_assert(kSkinnyThreads == 4 * kSkinnyRows, "one output per thread and reduction step");
 
+// C[m, n] as above for tall A: one thread per row over the whole of K, B staged
+// in shared memory (every lane reads the same entry), nothing to reduce.
+// Which of the two runs: skinny_row_threads.
+constexpr int kSkinnyChunkN = 64;  // K rows staged per step
+template <typename T, int NS>
+__global__ void __launch_bounds__(kSkinnyThreads) skinny_rows_kernel(
+    int M, int N, int K, C2<T> alpha, const C2<T>* __restrict__ A, int64_t lda,
+    const C2<T>* __restrict__ B, int64_t ldb, C2<T> beta, C2<T>* C, int64_t ldc) {
+  __shared__ C2<T> bs[kSkinnyChunkN][NS];
+  const int m = blockIdx.x * kSkinnyThreads + threadIdx.x;
+  const C2<T> zero = qeb::mk<T>(0, 0);
+  C2<T> acc[NS];
+#pragma unroll
+  for (int n = 0; n < NS; ++n) acc[n] = zero;
+  const C2<T>* arow = A + (m < M ? m : 0);
+  for (int k0 = 0; k0 < K; k0 += kSkinnyChunkN) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < NS * kSkinnyChunkN; i += kSkinnyThreads) {
+      const int n = i / kSkinnyChunkN, kk = i - n * kSkinnyChunkN;
+      const int k = k0 + kk;
+      bs[kk][n] = (n < N && k < K) ? B[k + (int64_t)n * ldb] : zero;
+    }
+    __syncthreads();
+    if (m < M) {
+      const int kn = min(kSkinnyChunkN, K - k0);
+#pragma unroll 8
+      for (int kk = 0; kk < kn; ++kk) {
+        const C2<T> a = arow[(int64_t)(k0 + kk) * lda];
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {
+          const C2<T> b = bs[kk][n];
+          acc[n].re = fma(a.re, b.re, acc[n].re);
+          acc[n].re = fma(-a.im, b.im, acc[n].re);
+          acc[n].im = fma(a.re, b.im, acc[n].im);
+          acc[n].im = fma(a.im, b.re, acc[n].im);
+        }
+      }
+    }
+  }
+  if (m >= M) return;
+  const bool use_beta = beta.re != T(0) || beta.im != T(0);
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    if (n >= N) break;
+    C2<T>* c = C + m + (int64_t)n * ldc;
+    C2<T> v = qeb::cmul(alpha, acc[n]);
+    if (use_beta) v = v + qeb::cmul(beta, *c);
+    *c = v;
+  }
+}
+
+// D = X^H Y as skinny_c_kernel computes it, for 9 to 16 narrow columns: one
+// warp per wide column, Y staged in shared memory for the eight columns of a
+// block.  Which of the two runs: skinny_c_plan.
+constexpr int kStagedWidth = 16;
+constexpr int kStagedChunk = 128;  // K rows staged per step
+template <typename T>
+__global__ void __launch_bounds__(kSkinnyThreads) skinny_staged_kernel(
+    int Mb, int Ns, int K, int krange, const C2<T>* __restrict__ X, int64_t ldx,
+    const C2<T>* __restrict__ Y, int64_t ldy, C2<T> alpha, C2<T> beta, C2<T>* C, int64_t ldc,
+    int swapped, C2<T>* __restrict__ P) {
+  constexpr int NS = kStagedWidth;
+  __shared__ C2<T> ys[NS][kStagedChunk];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int mb = blockIdx.x * kSkinnyWarps + warp;
+  const int kbeg = blockIdx.y * krange;
+  const int kend = min(K, kbeg + krange);
+  const C2<T> zero = qeb::mk<T>(0, 0);
+  C2<T> acc[NS];
+#pragma unroll
+  for (int n = 0; n < NS; ++n) acc[n] = zero;
+  const C2<T>* xcol = X + (int64_t)(mb < Mb ? mb : 0) * ldx;
+  for (int k0 = kbeg; k0 < kend; k0 += kStagedChunk) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < NS * kStagedChunk; i += kSkinnyThreads) {
+      const int n = i / kStagedChunk, kk = i - n * kStagedChunk;
+      const int k = k0 + kk;
+      ys[n][kk] = (n < Ns && k < kend) ? Y[k + (int64_t)n * ldy] : zero;
+    }
+    __syncthreads();
+    if (mb < Mb) {
+      C2<T> xv[kStagedChunk / 32];
+#pragma unroll
+      for (int j = 0; j < kStagedChunk / 32; ++j) {
+        const int k = k0 + lane + 32 * j;
+        xv[j] = (k < kend) ? xcol[k] : zero;
+      }
+#pragma unroll
+      for (int j = 0; j < kStagedChunk / 32; ++j) {
+        const int kk = lane + 32 * j;
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {
+          const C2<T> y = ys[n][kk];
+          // conj(x) * y
+          acc[n].re = fma(xv[j].re, y.re, acc[n].re);
+          acc[n].re = fma(xv[j].im, y.im, acc[n].re);
+          acc[n].im = fma(xv[j].re, y.im, acc[n].im);
+          acc[n].im = fma(-xv[j].im, y.re, acc[n].im);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      acc[n].re += __shfl_xor_sync(0xffffffffu, acc[n].re, off);
+      acc[n].im += __shfl_xor_sync(0xffffffffu, acc[n].im, off);
+    }
+  }
+  if (lane != 0 || mb >= Mb) return;
+  const bool use_beta = beta.re != T(0) || beta.im != T(0);
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    if (n >= Ns) break;
+    if (P != nullptr) {
+      P[(int64_t)blockIdx.y * Mb * Ns + mb + (int64_t)n * Mb] = acc[n];
+    } else {
+      C2<T> d = acc[n];
+      if (swapped) d.im = -d.im;
+      C2<T>* c = swapped ? C + n + (int64_t)mb * ldc : C + mb + (int64_t)n * ldc;
+      C2<T> v = qeb::cmul(alpha, d);
+      if (use_beta) v = v + qeb::cmul(beta, *c);
+      *c = v;
+    }
+  }
+}
+
 int g_sm_count = 0;
 
 int sm_count() {
@@ -670,16 +798,24 @@ int skinny_width(int n) {
 // side mb, the number of K slices (two waves of two blocks per SM, each slice
 // at least 1024 deep) and whether the warps of a block split K between them
 // (wk: when the blocks would not fill the GPU otherwise).
+//
+// `staged`: one warp per wide column with Y in shared memory, where the ring
+// kernel's blocks, whose 172 to 221 KB of ring let one run on an SM, fill
+// their last wave badly.  Measured, ring and staged: few steps per column for
+// many columns (300 x 900 x 16 complex128 21 and 11 us, 579 x 900 x 12 complex64
+// 15 and 11; 2400 x 900 x 13 complex128 43 and 47); 13 to 16 complex64 columns
+// against about a hundred long ones (80 725 x 97 x 16 91 and 64 us, 130 columns 117
+// and 95; 250 columns 195 and 194, 40 columns 42 and 41; complex128 126 and 169).
 struct SkinnyC {
-  bool use = false, swapped = false;
+  bool use = false, swapped = false, staged = false;
   int mb = 0, ns = 0, splits = 1, wk = 1;
   int groups() const {  // blocks along the large side
-    const int per = skinny_cols(skinny_width(ns)) * (kSkinnyWarps / wk);
+    const int per = staged ? kSkinnyWarps : skinny_cols(skinny_width(ns)) * (kSkinnyWarps / wk);
     return (mb + per - 1) / per;
   }
 };
 
-SkinnyC skinny_c_plan(int M, int N, int K) {
+SkinnyC skinny_c_plan(int M, int N, int K, bool single) {
   SkinnyC p;
   if (N <= kSkinnyMax) {
     p.use = true, p.mb = M, p.ns = N;
@@ -689,6 +825,14 @@ SkinnyC skinny_c_plan(int M, int N, int K) {
     return p;
   }
   const int by_depth = K / 1024 < 1 ? 1 : K / 1024;
+  p.staged = (p.ns > 8 && p.mb >= 512 && K <= 1536) ||
+             (single && p.ns > 12 && p.mb >= 64 && p.mb <= 192 && K >= 16384);
+  if (p.staged) {
+    const int want = (4 * sm_count() + p.groups() - 1) / p.groups();
+    p.splits = want < by_depth ? want : by_depth;
+    if (p.splits > 64) p.splits = 64;
+    return p;
+  }
   if ((int64_t)p.groups() * by_depth < 2 * sm_count()) p.wk = kSkinnyWarps;
   const int fill = 4 * sm_count() / p.groups();
   // a split product needs a second launch: not for the depth one block
@@ -714,6 +858,9 @@ int launch_skinny_c(const SkinnyC& p, bool wide, int K, int krange, const C2<T>*
                                                    C, ldc, sw, partials);
     return QEB_OK;
   };
+  if constexpr (NS > 8) {
+    if (p.staged) return launch(skinny_staged_kernel<T>, 0);
+  }
   if (p.wk > 1)
     return wide ? launch(skinny_c_kernel<T, NS, V, kSkinnyWarps>, skinny_c_smem<T, NS, V>())
                 : launch(skinny_c_kernel<T, NS, 1, kSkinnyWarps>, skinny_c_smem<T, NS, 1>());
@@ -750,7 +897,7 @@ template <typename T>
 int gemm_skinny_c(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, const C2<T>* B,
                   int64_t ldb, C2<T> be, C2<T>* C, int64_t ldc, void* scratch,
                   int64_t scratch_bytes, cudaStream_t stream) {
-  SkinnyC p = skinny_c_plan(M, N, K);
+  SkinnyC p = skinny_c_plan(M, N, K, sizeof(T) == 4);
   const int64_t slice_bytes = (int64_t)p.mb * p.ns * (int64_t)sizeof(C2<T>);
   if (p.splits > 1) {
     const int64_t fit = (scratch == nullptr) ? 0 : scratch_bytes / slice_bytes;
@@ -783,9 +930,70 @@ int gemm_skinny_c(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, co
   return qeb::cuda_status(cudaGetLastError(), "zgemm skinny launch");
 }
 
+// Whether an OP_N product runs with one thread per row instead of a K range per
+// warp: from some number of rows on, because blocks of 256 rows then fill the
+// GPU, sooner the shorter K is (a block's reduction over its warps costs as
+// much as a few K steps) and the wider the narrow side (its values, loaded
+// from global memory for every two rows, take over).  The table holds those
+// rows in thousands by width of the narrow side and by K, from timings of both
+// over 14 000 to 80 725 rows, 2 to 900 K values and 1 to 16 columns.  Range per warp
+// and thread per row: 80 725 x 600 x 8 complex128 563 and 305 us, 80 725 x 256 x 16
+// complex64 187 and 107, 23 847 x 17 x 13 complex64 13 and 9; on the other side 80 725
+// x 600 x 5 complex64 (93 and 145 us) and 6000 x 97 x 16 complex128 (13 and 29).  On either
+// side the choice is within a fifth of the faster one.
+bool skinny_row_threads(int M, int N, int K, bool single) {
+  constexpr int kNever = 1 << 30;
+  // from 28 000 rows on, when the last wave of one block per SM is three
+  // quarters full: the blocks of an SM share its FP64 pipe (256 K values, 16
+  // complex128 columns, range per warp and thread per row: 34 000 rows 115 and
+  // 94 us, 45 000 rows 145 and 180)
+  constexpr int kFullWaves = -1;
+  constexpr int kWidths[] = {2, 3, 4, 5, 6, 7, 8, 10, 12, 16};  // columns up to
+  constexpr int kDepths[] = {10, 24, 48, 150};                  // K up to, and above
+  constexpr int kRows[2][10][5] = {
+      {{28, kNever, kNever, kNever, kNever},  // complex128
+       {36, 42, 50, kNever, kNever},
+       {28, 36, 42, 58, 65},
+       {20, 36, 65, kNever, kNever},
+       {16, 20, 28, 50, 65},
+       {16, 20, 28, 28, 50},
+       {16, 20, 20, 28, 36},
+       {16, 20, kFullWaves, kFullWaves, kNever},
+       {16, 20, 20, 20, 20},
+       {16, 16, 20, kFullWaves, kFullWaves}},
+      {{65, 50, kNever, kNever, kNever},  // complex64
+       {20, 36, 42, 50, 75},
+       {28, 28, 28, 50, kNever},
+       {28, 28, 50, kNever, kNever},
+       {28, 20, 28, 65, kNever},
+       {20, 20, 20, 36, 36},
+       {28, 20, 20, 20, 28},
+       {20, 20, 50, kNever, kNever},
+       {16, 20, 16, 20, 28},
+       {16, 16, 16, 20, 28}}};
+  int w = 0, d = 0;
+  while (w < 9 && N > kWidths[w]) ++w;
+  while (d < 4 && K > kDepths[d]) ++d;
+  const int rows = kRows[single ? 1 : 0][w][d];
+  if (rows == kFullWaves) {
+    const int64_t blocks = ((int64_t)M + kSkinnyThreads - 1) / kSkinnyThreads;
+    const int64_t waves = (blocks + sm_count() - 1) / sm_count();
+    return M >= 28000 && 4 * blocks >= 3 * waves * sm_count();
+  }
+  return M / 1000 >= rows;
+}
+
 template <typename T>
 int gemm_skinny_n(int M, int N, int K, C2<T> al, const C2<T>* A, int64_t lda, const C2<T>* B,
                   int64_t ldb, C2<T> be, C2<T>* C, int64_t ldc, cudaStream_t stream) {
+  if (skinny_row_threads(M, N, K, sizeof(T) == 4)) {
+    auto* kernel = N <= 4 ? skinny_rows_kernel<T, 4>
+                          : (N <= 8 ? skinny_rows_kernel<T, 8> : skinny_rows_kernel<T, 16>);
+    const unsigned blocks = (unsigned)(((int64_t)M + kSkinnyThreads - 1) / kSkinnyThreads);
+    kernel<<<blocks, kSkinnyThreads, 0, stream>>>(M, N, K, al, A, lda, B, ldb, be, C, ldc);
+    qeb::count_launches(1);
+    return qeb::cuda_status(cudaGetLastError(), "zgemm skinny launch");
+  }
   const dim3 grid((M + kSkinnyRows - 1) / kSkinnyRows);
   const bool wide = sizeof(T) == 4 && wide_loads(A, lda);
   with_width(N, [&](auto w) {
@@ -916,7 +1124,7 @@ extern "C" int64_t qeb_zgemm_scratch_bytes(int opa, int M, int N, int K, int pre
   if (opa != QEB_OP_C || M <= 0 || N <= 0 || K <= 0) return 0;
   const int64_t elem = (precision == QEB_F64) ? 16 : 8;
   if (N <= kSkinnyMax || M <= kSkinnyMax) {
-    const SkinnyC p = skinny_c_plan(M, N, K);
+    const SkinnyC p = skinny_c_plan(M, N, K, precision != QEB_F64);
     return p.splits > 1 ? (int64_t)p.splits * p.mb * p.ns * elem : 0;
   }
   const int splits =
