@@ -74,7 +74,8 @@ int qeb_local_plan_create(qeb_local_plan** plan, int nx, int ny, int nz, int64_t
 int qeb_local_plan_destroy(qeb_local_plan* plan);
 /* info[0..7] = nx, ny, nz, npw, sticks, active y rows, precision, device;
  * with n >= 9, info[8] = blocks at each end of x and y that the compile-time
- * plane kernel keeps (0: run-time plane kernel). */
+ * plane kernel keeps (0: another kernel runs); with n >= 10, info[9] = 1 for
+ * line transforms, 0 for the generic kernels. */
 int qeb_local_plan_info(const qeb_local_plan* plan, int64_t* info, int n);
 /* Bytes of caller scratch needed for nbands (the stick buffer
  * nbands*nz*sticks complex values); the role of the grid scratch argument

@@ -396,14 +396,16 @@ class LocalPotentialWorkspace:
                 self.plane_waves, slots64.ctypes.data, self._code,
             )
         _lib.check("qeb_local_plan_create", status)
-        info = np.zeros(9, dtype=np.int64)
+        info = np.zeros(10, dtype=np.int64)
         _lib.check("qeb_local_plan_info",
-                   lib.qeb_local_plan_info(self._plan, info.ctypes.data, 9))
+                   lib.qeb_local_plan_info(self._plan, info.ctypes.data, 10))
         self.stick_count = int(info[4])
         self.active_rows = int(info[5])
         # blocks at each end of x and y that the compile-time plane kernel of a
-        # square plane keeps (qeb_local_plan.line_k), 0 for the run-time kernel
+        # square plane keeps (qeb_local_plan.line_k), 0 when another kernel runs
         self.pruned_plane = int(info[8])
+        # whether the passes are line transforms (else the generic kernels)
+        self.line_passes = bool(info[9])
         self._potential_cache: tuple | None = None
         self._kinetic_cache: tuple | None = None
         # When a list, each apply batch appends its (A, B, C) pass times in ms.

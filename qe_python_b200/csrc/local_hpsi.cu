@@ -452,16 +452,30 @@ extern "C" int qeb_local_plan_create(qeb_local_plan** out, int nx, int ny, int n
       p->xmask |= 1u << (x / x2);
       p->ymask |= 1u << (y / y2);
     }
-    if (nx == ny && !(prune_env && prune_env[0] == '0')) p->line_k = qeb::line_keep(nx, reach);
-    if (p->line_k > 0) {
-      p->xmask = 0;
-      for (int i = 0; i < x1; ++i)
-        if (i < p->line_k || i >= x1 - p->line_k) p->xmask |= 1u << i;
-      p->ymask = p->xmask;
-    }
-    std::vector<int> row(nx, -1);
-    for (int x = 0; x < nx; ++x)
-      if ((p->xmask >> (x / x2)) & 1u) row[x] = p->line_rows++;
+    // the plane's rows for k blocks at each end of x and y, or for the occupied
+    // blocks (k = 0); false: they do not fit shared memory
+    const uint32_t xmask = p->xmask, ymask = p->ymask;
+    std::vector<int> row(nx);
+    auto fits = [&](int k) {
+      p->line_k = k;
+      p->xmask = xmask;
+      p->ymask = ymask;
+      if (k > 0) {
+        p->xmask = 0;
+        for (int i = 0; i < x1; ++i)
+          if (i < k || i >= x1 - k) p->xmask |= 1u << i;
+        p->ymask = p->xmask;
+      }
+      p->line_rows = 0;
+      for (int x = 0; x < nx; ++x)
+        row[x] = ((p->xmask >> (x / x2)) & 1u) ? p->line_rows++ : -1;
+      p->line_columns = qeb::line_columns(p);
+      return p->line_columns > 0;
+    };
+    const int keep =
+        nx == ny && !(prune_env && prune_env[0] == '0') ? qeb::line_keep(nx, reach) : 0;
+    p->lines = keep > 0 && fits(keep);
+    if (!p->lines) p->lines = fits(0);
     stick_map.assign((size_t)ny * p->line_rows, -1);
     for (int s = 0; s < nst; ++s)
       stick_map[(size_t)(sticks[s] / nx) * p->line_rows + row[sticks[s] % nx]] = s;
@@ -470,8 +484,6 @@ extern "C" int qeb_local_plan_create(qeb_local_plan** out, int nx, int ny, int n
       entry_pos[e] = entry_stick[e] % 32 * (nz | 1) + entry_z[e];
       p->zmask |= 1u << (entry_z[e] / z2);
     }
-    p->line_columns = qeb::line_columns(p);
-    p->lines = p->line_columns > 0;
   }
   int rc = QEB_OK;
   if (p->lines && ((rc = upload(&p->stick_map, stick_map)) ||
@@ -534,6 +546,7 @@ extern "C" int qeb_local_plan_info(const qeb_local_plan* p, int64_t* info, int n
   info[6] = p->precision;
   info[7] = p->device;
   if (n >= 9) info[8] = p->line_k;
+  if (n >= 10) info[9] = p->lines ? 1 : 0;
   return QEB_OK;
 }
 

@@ -28,7 +28,8 @@ struct qeb_local_plan {
   // Static plane kernel of square planes whose sticks all lie in
   // [0, line_k n2) or [n - line_k n2, n) of x and y: the plane holds the rows
   // of those 2 line_k blocks of x.  0: run-time kernel, the blocks of the
-  // masks below.  QEB_PRUNE_PLANE=0 keeps a plan on the run-time kernel.
+  // masks below, also where the rows of all 2 line_k blocks exceed shared
+  // memory (FP64, 192 points).  QEB_PRUNE_PLANE=0 keeps a plan on it.
   int line_k;
   int line_rows;     // rows (x values) the plane holds
   int line_columns;  // columns per batch of the run-time kernel

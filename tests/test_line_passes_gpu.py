@@ -67,8 +67,21 @@ def test_every_length(cuda_device, n, precision):
     as ecutrho = 4 ecutwfc makes it), z lines of another one."""
     nz = LENGTHS[(LENGTHS.index(n) * 7 + 3) % len(LENGTHS)] if n <= 96 else 20
     # (FP64 planes of wider spheres are refused from 160 points on)
-    _check((n, n, nz), _basis((n, n, nz), 0.47 if n < 160 else 0.28, n), precision,
-           density=n <= 96)
+    fraction = 0.47 if n < 160 else (0.28 if n < 192 else 0.24)
+    ws = _check((n, n, nz), _basis((n, n, nz), fraction, n), precision, density=n <= 96)
+    # the static kernel's rows of 192 FP64 points exceed shared memory: run-time kernel
+    assert ws.line_passes and (ws.pruned_plane > 0) == ((n, precision) != (192, "f64"))
+
+
+@pytest.mark.parametrize("n,nz,fraction,precision,lines,kept", [
+    (192, 20, 0.24, "f64", True, 0),   # the occupied blocks' rows fit where the kept ones do not
+    (192, 20, 0.28, "f64", False, 0),  # neither fit: generic kernels, no blocks reported
+    (192, 20, 0.28, "f32", True, 4),
+    (64, 125, 0.47, "f64", False, 0),  # z without a split
+])
+def test_plane_layout(cuda_device, n, nz, fraction, precision, lines, kept):
+    ws = _check((n, n, nz), _basis((n, n, nz), fraction, 3), precision, density=False)
+    assert (ws.line_passes, ws.pruned_plane) == (lines, kept)
 
 
 @pytest.mark.parametrize("precision", ["f32", "f64"])
