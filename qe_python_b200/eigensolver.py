@@ -14,8 +14,8 @@ Several k points' solves, each a chain of small latency-bound kernels, then
 run side by side on the GPU; the host reads the error codes when it reads
 the eigenvalues.
 
-Small subspaces (SMALL_LIMIT) take one kernel of libqeb200.so instead of that
-chain.  ``ReducedSolve.launch`` enqueues a solve on a stream and returns at once;
+Small subspaces (qeb_small_eigh_max columns) take one kernel of libqeb200.so
+instead of that chain.  ``ReducedSolve.launch`` enqueues a solve on a stream and returns at once;
 ``ReducedSolve.result`` makes the current stream wait for it and returns the
 lowest ``roots`` pairs, or falls back to the canonical orthogonalisation of
 the overlap when S was not numerically positive definite.
@@ -34,9 +34,6 @@ from . import _lib
 
 _P, _I = ctypes.c_void_p, ctypes.c_int
 _MODE_VECTOR, _FILL_LOWER = 1, 0
-
-# Columns up to which the one-launch solver is the faster one.
-SMALL_LIMIT = 32
 
 _lock = threading.Lock()
 _state: dict = {}
@@ -118,7 +115,7 @@ def zheevd_async(matrix: torch.Tensor, stream: torch.cuda.Stream):
 class ReducedSolve:
     """One asynchronous solve of H c = e S c for the lowest ``roots`` pairs.
 
-    Subspaces of up to SMALL_LIMIT columns go to the one-launch kernel
+    Subspaces of up to qeb_small_eigh_max columns go to the one-launch kernel
     (qeb_small_generalized_eigh), larger ones, and those whose rotations did
     not converge, to the Cholesky reduction and zheevd."""
 
@@ -132,7 +129,7 @@ class ReducedSolve:
         """Enqueue the solve of the Hermitian pair (h, s) on the stream after
         the work the current stream has enqueued so far."""
         n = h.shape[0]
-        if n <= SMALL_LIMIT and 1 <= roots <= n and all(
+        if n <= _lib.load().qeb_small_eigh_max() and 1 <= roots <= n and all(
                 m.dtype == torch.complex128 and m.is_cuda and m.stride(1) == 1 and m.stride(0) >= n
                 for m in (h, s)):
             self._launch_small(h, s, roots)
