@@ -62,14 +62,57 @@ def test_degenerate_diagonal_and_scaled(cuda_device):
         assert np.max(np.abs(e - want)) <= 1e-13 * np.abs(want).max()
 
 
-def test_indefinite_overlap_takes_the_canonical_route(cuda_device):
+def _status(h, s, roots):
+    """What the one-launch solver reports of the pencil."""
+    import torch
+
+    from qe_python_b200 import _lib
+
+    n = h.shape[0]
+    hd, sd = (torch.from_numpy(np.ascontiguousarray(m)).cuda() for m in (h, s))
+    values = torch.zeros(roots + 1, dtype=torch.float64, device="cuda")
+    vectors = torch.zeros((roots, n), dtype=torch.complex128, device="cuda")
+    _lib.check("qeb_small_generalized_eigh", _lib.load().qeb_small_generalized_eigh(
+        n, roots, hd.data_ptr(), n, sd.data_ptr(), n, values.data_ptr(), vectors.data_ptr(), n,
+        int(torch.cuda.current_stream().cuda_stream)))
+    return values.cpu().numpy()[roots]
+
+
+def _with_smallest(smallest):
+    """A pencil whose overlap has one eigenvalue ``smallest`` and nine ones."""
     h, s = _pencil(10, 3)
     u = np.linalg.qr(s)[0]
-    s = u @ np.diag([1e-18 * -1] + [1.0] * 9) @ u.conj().T
-    s = 0.5 * (s + s.conj().T)
+    weights = np.array([smallest] + [1.0] * 9)
+    s = (u * weights) @ u.conj().T
+    return h, 0.5 * (s + s.conj().T), u
+
+
+def test_indefinite_overlap_takes_the_canonical_route(cuda_device):
+    h, s, u = _with_smallest(-1e-6)
+    assert 1 <= _status(h, s, 4) <= 10  # the Cholesky factorisation fails
     e, c = _solve(h, s, 4)
-    assert np.max(np.abs(h @ c - (s @ c) * e)) > 0 and np.all(np.diff(e) >= 0)
-    assert np.max(np.abs(c.conj().T @ s @ c - np.eye(4))) <= 1e-8
+    # the pencil on the nine directions that are left, where S is the identity
+    kept = u[:, 1:]
+    want = np.linalg.eigvalsh(kept.conj().T @ h @ kept)[:4]
+    scale = np.linalg.norm(h, 2)
+    tol = 40 * 10 * 2.2e-16
+    assert np.max(np.abs(e - want)) <= tol * scale
+    assert np.max(np.abs(c.conj().T @ s @ c - np.eye(4))) <= 10 * tol
+    assert np.max(np.abs(u[:, :1].conj().T @ c)) <= 10 * tol  # nothing of the dropped one
+    residual = kept.conj().T @ (h @ c - (s @ c) * e)
+    assert np.max(np.abs(residual)) <= 10 * tol * scale
+
+
+def test_nearly_singular_overlap_stays_on_its_route(cuda_device):
+    import scipy.linalg
+
+    h, s, u = _with_smallest(1e-8)
+    assert _status(h, s, 4) == 0.0
+    e, c = _solve(h, s, 4)
+    # backward error n eps of L^-1 H L^-H, whose norm is that of H over 1e-8
+    tol = 40 * 10 * 2.2e-16 * np.linalg.norm(h, 2) * 1e8
+    assert np.max(np.abs(e - scipy.linalg.eigh(h, s, eigvals_only=True)[:4])) <= tol
+    assert np.max(np.abs(c.conj().T @ s @ c - np.eye(4))) <= 40 * 10 * 2.2e-16 * 1e8
 
 
 @pytest.mark.parametrize("dtype", ["complex64", "complex128"])
