@@ -19,6 +19,9 @@ void set_error(const char* fmt, ...) {
 
 int cuda_status(cudaError_t err, const char* where) {
   if (err == cudaSuccess) return QEB_OK;
+  // the error is reported here: left as the thread's last error, the caller's
+  // next unrelated check would report it again
+  cudaGetLastError();
   set_error("%s: %s", where, cudaGetErrorString(err));
   return QEB_ECUDA;
 }
