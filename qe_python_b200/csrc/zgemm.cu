@@ -759,13 +759,17 @@ int choose_splits(int M, int N, int K) {
 // (23 847 x 184 x 184: 32 x 32 243 us, 48 x 48 260; 80 725 x 97 x 300: 32 x 32 804,
 // 64 x 64 957), A^H B a little faster in large ones, which load less per product
 // (512 x 256 x 11 019: 64 x 64 370 us, 32 x 32 385).  The rates only weigh the
-// terms against each other.
+// terms against each other.  No fewer slices than choose_splits: rounding grows
+// with the length of a chain of additions, and the fewer slices that are often
+// faster (512 x 256 x 6000 202 us, 263 so) doubled the error of narrow products
+// (512 x 40 x 11 019: 1.7e-15 relative, 8.7e-16 so).
 struct MmaPlan {
   int bm = 64, bn = 64, splits = 1;
 };
 
 MmaPlan mma_plan(int M, int N, int K, bool split) {
   constexpr double kSmRate = 30.0e3, kSliceBytes = 4.0e6;  // per SM; bytes per us
+  const int least = split ? choose_splits(M, N, K) : 1;
   MmaPlan best;
   double best_time = 0.0;
   for (int bm : {64, 48, 32})
@@ -773,7 +777,7 @@ MmaPlan mma_plan(int M, int N, int K, bool split) {
       const int64_t tiles = (int64_t)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
       const double rate = kSmRate * (split ? 1.0 - 0.4 / bm - 0.4 / bn
                                            : 1.0 - 0.05 * (bm * bn / 1024.0 - 1.0));
-      for (int s = 1; s <= (split ? 64 : 1) && (s == 1 || K / s >= 64); ++s) {
+      for (int s = least; s <= (split ? 64 : 1) && (s == least || K / s >= 64); ++s) {
         const int64_t per_sm = (tiles * s + sm_count() - 1) / sm_count();
         const int depth = ((K + s - 1) / s + kMmaK - 1) / kMmaK * kMmaK;
         double time = (double)per_sm * depth * bm * bn / rate;
