@@ -9,9 +9,9 @@
 #define QEB_LINE_LENGTHS(X)                                                            \
   X(16, 4, 4, 1, 1) X(18, 3, 6, 1, 1) X(20, 4, 5, 1, 1) X(24, 4, 6, 1, 1)              \
   X(25, 5, 5, 2, 2) X(27, 3, 9, 1, 1) X(30, 6, 5, 2, 2) X(32, 4, 8, 1, 1)              \
-  X(36, 4, 9, 1, 1) X(40, 8, 5, 2, 2) X(45, 9, 5, 2, 3) X(48, 8, 6, 2, 2)              \
+  X(36, 6, 6, 2, 2) X(40, 8, 5, 2, 2) X(45, 9, 5, 2, 3) X(48, 8, 6, 2, 2)              \
   X(50, 10, 5, 3, 3) X(54, 9, 6, 2, 3) X(60, 12, 5, 3, 3) X(64, 8, 8, 2, 2)            \
   X(72, 8, 9, 2, 2) X(75, 15, 5, 3, 4) X(80, 8, 10, 2, 2) X(81, 9, 9, 2, 3)            \
   X(90, 10, 9, 2, 3) X(96, 12, 8, 3, 3) X(100, 10, 10, 2, 3) X(108, 12, 9, 3, 3)       \
-  X(120, 12, 10, 3, 3) X(128, 16, 8, 4, 4) X(135, 15, 9, 3, 4) X(144, 16, 9, 4, 4)     \
+  X(120, 12, 10, 3, 3) X(128, 16, 8, 4, 4) X(135, 15, 9, 3, 4) X(144, 12, 12, 3, 3)     \
   X(150, 15, 10, 3, 4) X(160, 16, 10, 4, 4) X(180, 15, 12, 3, 4) X(192, 16, 12, 4, 4)
