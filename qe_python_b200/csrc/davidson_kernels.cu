@@ -87,21 +87,21 @@ __global__ void __launch_bounds__(kReduceThreads) column_reduce(
   const int64_t first = part * part_rows, last = min(rows, first + part_rows);
   const C2<T>* l = left + col * ldl;
   const C2<T>* r = MODE == 2 ? right + col * ldr : nullptr;
-  double re = 0.0, im = 0.0;
-  auto add = [&](int64_t g, C2<T> a, C2<T> b) {
+  double re2[2] = {0.0, 0.0}, im2[2] = {0.0, 0.0};  // of the even and the odd runs
+  auto add = [&](int c, int64_t g, C2<T> a, C2<T> b) {
     if (MODE == 2) {
-      re += (double)a.re * b.re + (double)a.im * b.im;
-      im += (double)a.re * b.im - (double)a.im * b.re;
+      re2[c] += (double)a.re * b.re + (double)a.im * b.im;
+      im2[c] += (double)a.re * b.im - (double)a.im * b.re;
     } else {
       const double m = (double)a.re * a.re + (double)a.im * a.im;
-      re += (MODE == 1) ? diag[g] * m : m;
+      re2[c] += (MODE == 1) ? diag[g] * m : m;
     }
   };
   constexpr int kStep = kReduceThreads * V;
   int64_t g = first + threadIdx.x * V;
   // four loads in flight per thread, two from each operand of an inner product
-  // (four from each took 160 us on 50 000 x 480 complex128, two 118), the
-  // sums in row order
+  // (four from each took 160 us on 50 000 x 480 complex128, two 118); two sums,
+  // half the chain of additions, make up for the longer parts
   constexpr int kRuns = MODE == 2 ? 2 : 4;
   for (; g + (kRuns - 1) * kStep + V <= last; g += kRuns * kStep) {
     C2<T> a[kRuns][V], b[kRuns][V];
@@ -113,10 +113,13 @@ __global__ void __launch_bounds__(kReduceThreads) column_reduce(
 #pragma unroll
     for (int u = 0; u < kRuns; ++u)
 #pragma unroll
-      for (int v = 0; v < V; ++v) add(g + u * kStep + v, a[u][v], MODE == 2 ? b[u][v] : a[u][v]);
+      for (int v = 0; v < V; ++v)
+        add(u & 1, g + u * kStep + v, a[u][v], MODE == 2 ? b[u][v] : a[u][v]);
   }
   for (; g < last; g += kStep)
-    for (int v = 0; v < V && g + v < last; ++v) add(g + v, l[g + v], MODE == 2 ? r[g + v] : l[g + v]);
+    for (int v = 0; v < V && g + v < last; ++v)
+      add(0, g + v, l[g + v], MODE == 2 ? r[g + v] : l[g + v]);
+  double re = re2[0] + re2[1], im = im2[0] + im2[1];
   re = block_sum(re, shared[0]);
   if (MODE == 2) im = block_sum(im, shared[1]);
   if (parts > 1) {
