@@ -92,8 +92,8 @@ def parse_args():
 
 
 # DRAM bytes (read + write) of one plane-pass launch of the 256-band
-# microbenchmark operator, from one ncu capture: 487.2 GB/s over 207.97 us.
-PASS_B_NCU_TRAFFIC = {("pass_b", 256): 101.33e6}
+# microbenchmark operator, from one ncu capture: 78.8 MB read, 22.2 MB written.
+PASS_B_NCU_TRAFFIC = {("pass_b", 256): 101.01e6}
 
 
 # How the SCF benchmark cells differ from the configurations they stand for:
@@ -710,7 +710,7 @@ def run_b200(args) -> None:
                     "algorithmic_bytes": amount,
                     "peak_source": peaks["source"],
                     "note": "pass B is bound by the shared-memory data path (ncu: LSU "
-                            "wavefronts 82 %, issue 71 % active), not by HBM"}
+                            "wavefronts 84 %, issue 70 % active), not by HBM"}
         if dominant == "pass_b":
             roofline["fp32_fft_rate"] = plane_fft_rate(work.shape, nb, seconds)
     elif dominant in ("calbec_gemm", "add_gemm") and forms["mixed"][1].tensor_gemm:

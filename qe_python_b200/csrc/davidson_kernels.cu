@@ -74,7 +74,7 @@ __device__ __forceinline__ double cluster_read(const double* p, unsigned rank) {
 // reads: one block per column left 131 blocks on 148 SMs for the corrections
 // of the 216-atom cell (80 725 x 131 complex64: 57 us, 1.5 TB/s).  With the
 // column kernels below: g_psi, norms and normalisation of that block 0.173 ->
-// 0.085 ms.
+// 0.087 ms.
 template <typename T, int MODE, int V>
 __global__ void __launch_bounds__(kReduceThreads) column_reduce(
     int64_t rows, int parts, int64_t part_rows, const C2<T>* __restrict__ left, int64_t ldl,

@@ -21,9 +21,12 @@
 //     contiguous,
 //   * twiddle reads are broadcasts from tables laid out [role][k].
 // The steps of one transform are separated by block barriers; several blocks
-// per SM fill them.  The passes are bound by instruction issue and the
-// shared-memory data path together (64 x 64 plane, FP32: 71 % and 82 %), FP64
-// planes of 135 points by one resident block's latency.  Measured against
+// per SM fill them.  The plane pass is bound by the shared-memory data path
+// (share of its wavefronts: 64 x 64 FP32 84 %, FP64 91 %, 135 x 135 FP32 72 %) with
+// issue next (70, 41 and 66 %); FP64 planes of 135 points by neither (60 and
+// 34 %): one block of 16 warps fits an SM and waits at its barriers.  The z passes
+// wait for their gathered entries and barriers (52 to 67 % of the wavefronts).
+// Measured against
 // lines spread over the lanes of a warp, plane pass: 135^3 of 96 bands FP32
 // 1.313 -> 0.887 ms, FP64 2.627 -> 1.866; 90^3 of 200 bands FP32 0.697 ->
 // 0.520; 64^3 of 256 bands FP32 0.209 -> 0.197, FP64 0.383 -> 0.352; z passes

@@ -751,9 +751,10 @@ int skinny_width(int n) {
 }
 
 // Skinny OP_C plan: the narrow side (N, else M when N is wide), the large
-// side mb, the number of K slices (two waves of two blocks per SM, each slice
-// at least 1024 deep) and whether the warps of a block split K between them
-// (wk: when the blocks would not fill the GPU otherwise).
+// side mb, the number of K slices (up to four blocks per SM in all, each slice
+// at least 1024 deep; by whole waves for 9 to 16 columns against few) and whether
+// the warps of a block split K between them (wk: when the blocks would not fill
+// the GPU otherwise).
 struct SkinnyC {
   bool use = false, swapped = false;
   int mb = 0, ns = 0, splits = 1, wk = 1;

@@ -215,7 +215,10 @@ class _DeviceProjectors:
 # than the overlap gains.  Measured, side stream against one stream: 8 bands of
 # 579 plane waves, 8 channels (4e4) 103 and 59 us; 24 bands of the 8-atom cell
 # (2e6) 98 and 65; 4 bands of the 64-atom cell (2e7) FP64 105 and 134; 37 bands
-# of a slab (6e7) 161 and 179.
+# of a slab (6e7) 161 and 179.  The count alone does not decide above the line:
+# the side stream is the slower one for 4 bands of the 64-atom cell in FP32 (98
+# and 70), 16 bands on 64^3 in FP32 (112 and 93) and 1 band of the 216-atom cell
+# in FP64 (469 and 407), which keep it.
 OVERLAP_MIN_MACS = 1 << 24
 
 

@@ -1,8 +1,8 @@
-"""Four-step and generic FFT kernels on the benchmark grids (GPU).
+"""Line-transform and generic FFT kernels on the benchmark grids (GPU).
 
 The 90^3 and 135^3 grids of the 64- and 216-atom cells run through the
-four-step register kernels; the same operator with QEB_FORCE_GENERIC=1 set at
-plan creation runs the generic Stockham kernels.  Both must agree with the
+line transforms; the same operator with QEB_FORCE_GENERIC=1 set at plan
+creation runs the generic Stockham kernels.  Both must agree with the
 oracle (apply_serial, qepy_pw/_native_fft.pyx:2338-2455) to 1e-12 (FP64).
 """
 
@@ -95,10 +95,9 @@ FOUR_STEP_LENGTHS = (16, 24, 32, 36, 48, 64, 72, 90, 96, 108, 128, 135, 144, 180
 
 @pytest.mark.parametrize("n", FOUR_STEP_LENGTHS)
 def test_every_four_step_length(cuda_device, n):
-    """Each listed four-step length (cubic n^3 grid, G sphere of radius n/6)
-    in both precisions against the oracle, the factor pairs with an odd N2
-    (8 x 9, 9 x 15, 12 x 15) included: their line groups exchange through a
-    buffer of stride N2."""
+    """Cubic n^3 grids (G sphere of radius n/6) in both precisions against the
+    oracle, over lines of two power-of-two factors, of an odd factor (8 x 9,
+    15 x 9, 15 x 12) and of two equal ones (6 x 6, 8 x 8, 12 x 12)."""
     import torch
 
     length = 10.0

@@ -1,14 +1,14 @@
-"""The pruned plane pass of the 64-point four-step planes.
+"""The compile-time plane kernel of 64-point planes beside the run-time one.
 
 When every stick of a plan lies within the rows and columns [0, 16) and
-[48, 64) of a 64 x 64 plane (K = 2 blocks of N2 = 8 at each end), pass B
-keeps only those 32 rows and skips the D1 blocks 2..5 that are zero on input
-to the inverse line transforms and unread after the forward ones.  Every
-step adds or multiplies the same values as the active-row plane pass, so the
-two give the same output bit for bit (QEB_PRUNE_PLANE=0 builds a plan on
-the active-row plane).  Both are checked against the oracle's apply_serial
+[48, 64) of a 64 x 64 plane (two blocks of eight at each end), the plane pass
+runs a kernel compiled for those 32 rows, which skips the blocks that are zero
+on input to the inverse line transforms and unread after the forward ones.
+Every step adds or multiplies the same values as the run-time kernel, so the
+two give the same output bit for bit (QEB_PRUNE_PLANE=0 keeps a plan on the
+run-time kernel).  Both are checked against the oracle's apply_serial
 (qepy_pw/_native_fft.pyx:2338-2455); a basis whose sticks reach past the
-kept rows stays on the active-row plane.
+kept rows stays on the run-time kernel.
 """
 
 from __future__ import annotations
@@ -87,7 +87,7 @@ def test_sticks_past_the_kept_rows_use_the_active_row_plane(cuda_device):
 @pytest.mark.parametrize("precision", ["f32", "f64"])
 def test_pruned_plane_in_a_k_point_batch(cuda_device, monkeypatch, precision):
     """Several k points in one launch per pass (qeb_apply_local_multi), each
-    with its own slot tables: the same bits as the active-row plane batch."""
+    with its own stick map: the same bits as a batch on the run-time kernel."""
     import torch
 
     from qe_python_b200.basis import apply_local_multi
@@ -112,7 +112,7 @@ def test_pruned_plane_in_a_k_point_batch(cuda_device, monkeypatch, precision):
         local = np.random.default_rng(24)
         vectors, targets, kinetics = [], [], []
         for i, b in enumerate(bases):
-            nb = 3 + i  # uneven band counts, odd and even (two bands per block)
+            nb = 3 + i  # uneven band counts, odd and even
             psi = local.standard_normal((len(b), nb)) + 1j * local.standard_normal((len(b), nb))
             vectors.append(to_device_f(psi, cdt, torch.device("cuda")))
             targets.append(empty_f(len(b), nb, cdt, torch.device("cuda")))
